@@ -86,11 +86,11 @@ def sample_workload(name: str):
 
 
 def algorithmic_bytes(case, precision: int = abi.PREC_FP64) -> float:
-    """Bytes one launch of the stage kernel must move per cell, averaged over the families and the RK
+    """Bytes one stage (its flux and cell kernels) must move per cell, averaged over the families and the RK
     stages: read U_(k-1) and U_0 and write U_k (24 nc, FP64 state); per direction the face normal and
     area (32) and the cell length (8) in FP64, or their single-precision copies (16 and 4) in the
-    FP32-flux form; the volume (8); the boundary map (4); in a coupled run the nine
-    frozen-gas values the fused source reads (72; 36 for their single-precision copy in the FP32-flux
+    FP32-flux form; the volume (8); in a coupled run the nine
+    frozen-gas values the source reads (72; 36 for their single-precision copy in the FP32-flux
     form) and the relaxation time it writes on the last stage (8 / nrk), or, for an evaporating family
     of a 2-D or 3-D run, the source its own kernel wrote (8 nc; 4 nc in single precision in the FP32-flux
     form); the local dt (8) in steady mode; in 1-D runs the sensor weight (8) when the shock detector
@@ -102,7 +102,7 @@ def algorithmic_bytes(case, precision: int = abi.PREC_FP64) -> float:
     geo = 20 if f32 else 40
     word = 4 if f32 else 8
     for f in case.families:
-        b = 24 * f.nc + geo * ndir + 8 + 4
+        b = 24 * f.nc + geo * ndir + 8
         if case.numerics.coupled:
             b += word * f.nc if (ndir >= 2 and f.evap != "none") else 9 * word + 8 / nrk
         if case.numerics.shock_detector and ndir == 1:
@@ -113,19 +113,10 @@ def algorithmic_bytes(case, precision: int = abi.PREC_FP64) -> float:
     return float(np.mean(per))
 
 
-# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per cell of one stage-kernel launch, from an
-# ncu capture of the 4-block case of the 48-block tree in the chosen form (second RK stage of each
-# family, 3,714,802 cells). The 48-block case is the same recipe with the same tile shapes, so its
-# launches move about the same bytes per cell: traffic per launch = these x its cells.
-DRAM_BYTES_PER_CELL = {"MK": 302.2, "IG": 333.0, "AG": 537.2}
-
-
 def dram_traffic(case, workload: str, precision: int):
-    """Measured DRAM bytes of one stage-kernel launch of the workload (mean over its families), where a
-    capture of the same recipe and form exists; None otherwise."""
-    if not workload.startswith("multiblock") or precision != abi.PREC_FP32FLUX:
-        return None
-    return float(np.mean([DRAM_BYTES_PER_CELL[f.closure] for f in case.families])) * case.ncells
+    """Measured DRAM bytes of one stage of the workload (mean over its families), where a capture of the same
+    recipe and form exists; None otherwise."""
+    return None
 
 
 class Clocks:
@@ -444,12 +435,12 @@ def run_ours(args, rank, world, dist):
         traffic = dram_traffic(case, args.workload, prec)
         extra = {
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                         "traffic": traffic, "traffic_unit": "bytes per launch (ncu DRAM read + write)",
+                         "traffic": traffic, "traffic_unit": "bytes per stage (ncu DRAM read + write)",
                          "algorithmic_bytes_per_launch": bpc * cells,
-                         "kernel": "k_stage3", "bytes_per_cell": bpc,
+                         "kernel": "k_flux + k_cells", "bytes_per_cell": bpc,
                          "launch_ms": stage_ms,
                          "note": f"peak of {peak_kind}; achieved = algorithmic bytes per launch / mean CUDA-event "
-                                 f"duration of the stage kernel's launches"},
+                                 f"duration of a stage's flux and cell kernels"},
             "plain_fp64": {"value": plain_rate, "unit": "cell-updates/s"} if plain_rate else None,
             "chosen_vs_plain": (value / world / plain_rate) if plain_rate else None,
             "l1_error_vs_plain": l1,

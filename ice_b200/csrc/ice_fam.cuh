@@ -1,6 +1,6 @@
 // ice_fam.cuh -- the launcher of one family's RK stage, templated on its closure and Riemann
-// solver: ghost layers, sensor, connection and boundary fluxes, then the stage kernel of the
-// closure and precision (ice_stage.cuh), and the IRS sweeps when they are on.
+// solver: ghost layers, sensor, fluxes of the boundary records (in the plain form of every face),
+// then the stage kernel of the closure and precision (ice_stage.cuh), and the IRS sweeps when they are on.
 #pragma once
 #include "ice_kernels.cuh"
 #include "ice_mlp.cuh"
@@ -14,11 +14,18 @@ template <int CL> inline void launch_stage_of(const LaunchArgs& a, bool write_r)
   else { if (f32) launch_stage_ag_f32(a, write_r); else launch_stage_ag_f64(a, write_r); }
 }
 
-template <int CL> inline void launch_bound_of(const LaunchArgs& a) {
+template <int CL> inline void launch_flux_of(const LaunchArgs& a) {
   const bool f32 = a.precision == ICE_PREC_FP32FLUX && !a.irs;
-  if constexpr (CL == MK) { if (f32) launch_bound_mk_f32(a); else launch_bound_mk_f64(a); }
-  else if constexpr (CL == IG) { if (f32) launch_bound_ig_f32(a); else launch_bound_ig_f64(a); }
-  else { if (f32) launch_bound_ag_f32(a); else launch_bound_ag_f64(a); }
+  if constexpr (CL == MK) { if (f32) launch_flux_mk_f32(a); else launch_flux_mk_f64(a); }
+  else if constexpr (CL == IG) { if (f32) launch_flux_ig_f32(a); else launch_flux_ig_f64(a); }
+  else { if (f32) launch_flux_ag_f32(a); else launch_flux_ag_f64(a); }
+}
+
+template <int CL> inline void launch_beta_of(const LaunchArgs& a) {
+  const bool f32 = a.precision == ICE_PREC_FP32FLUX && !a.irs;
+  if constexpr (CL == MK) { if (f32) launch_beta_mk_f32(a); else launch_beta_mk_f64(a); }
+  else if constexpr (CL == IG) { if (f32) launch_beta_ig_f32(a); else launch_beta_ig_f64(a); }
+  else { if (f32) launch_beta_ag_f32(a); else launch_beta_ag_f64(a); }
 }
 
 template <int CL> inline void launch_source_of(const LaunchArgs& a) {
@@ -34,14 +41,16 @@ void launch_family_t(const LaunchArgs& a) {
   cudaStream_t s = a.s;
   auto tick = [&](int cls) { if (a.tick) a.tick(a.tick_ctx, cls, s); };
   auto grid = [](long long n, int t) { return (unsigned)((n + t - 1) / t); };
-  // compute_source comes first in the stage (Mod_Explicit.f90:111-117). The staged stage kernel
-  // evaluates it per cell itself for a family without evaporation; an evaporating family's source
+  const bool f32 = a.precision == ICE_PREC_FP32FLUX && !a.irs;
+  // compute_source comes first in the stage (Mod_Explicit.f90:111-117). In the FP32-flux form the cells'
+  // kernel evaluates the source of a family without evaporation itself; an evaporating family's source
   // (iterative, with lane-divergent trip counts) runs in its own kernel at full occupancy, or in the
-  // surrogate's source kernel, and the stage kernel reads it (FamDev::src_ready)
+  // surrogate's source kernel, and the stage reads it (FamDev::src_ready). So does every FP64 source, whose
+  // deterministic elementary functions would take the cells' kernel's registers, and the plane kernel's.
   if (a.F.coupled && a.mlp_img) {
     launch_source_mlp(CL, a, a.mlp_img, *a.mlp_norm);
     tick(KC_SOURCE);
-  } else if (a.F.coupled && (a.ntile3 == 0 || a.F.src_ready)) {
+  } else if (a.F.coupled && (a.F.src_ready || !f32 || a.plane)) {
     launch_source_of<CL>(a);
     tick(KC_SOURCE);
   }
@@ -55,17 +64,13 @@ void launch_family_t(const LaunchArgs& a) {
     }
     tick(KC_GHOST);
   }
-  // the Jameson sensor: the staged stage kernel and the boundary kernels evaluate it from the
-  // density they read; only the 1-D stage kernel reads it from a field
-  if (a.sd && a.ntile3 == 0) {
-    k_beta<<<grid(a.G.NI, 256), 256, 0, s>>>(a.G, a.F);
+  if (a.sd) {                                  // the Jameson sensor
+    launch_beta_of<CL>(a);
     tick(KC_BETA);
   }
   if (a.xchg) a.xchg(a, ICE_GPU_HALO_BETA);    // the weights of partner cells another rank steps
-  if (a.nown > 0 || a.nbc > 0 || a.xchg) {
-    launch_bound_of<CL>(a);
-    tick(KC_BOUND);
-  }
+  launch_flux_of<CL>(a);
+  tick(a.plane ? KC_BOUND : KC_STAGE);         // (else the interior faces come with the records)
   if (!a.irs) {
     launch_stage_of<CL>(a, false);
     tick(KC_STAGE);

@@ -9,17 +9,18 @@
 //   (k_empty_scan, k_empty_apply for a family with the coupler's imports: Mod_dt.f90:134-242)
 //   k_time         dtglobal, time += dt                               (Mod_Explicit.f90:67-73)
 //   per family, per RK stage:
-//     k_source     the source of an evaporating family (or a 1-D run), or the surrogate's
-//                  k_source_mlp                                        (Mod_Sources.f90:465-622)
+//     k_source     the source (plain form; an evaporating family of the FP32-flux form; 1-D runs), or the
+//                  surrogate's k_source_mlp                            (Mod_Sources.f90:465-622)
+//     (in the FP32-flux form's 1-D runs k_rec and k_stage take the place of k_flux and k_cells)
 //     k_ghost      both ghost layers from the record list (two launches, layer 1 then
 //                  layer 2, where a block is one cell deep along a record's face), block
 //                  connections as on-device copies in one HBM pool    (Lib_Ghost.f90:29-387)
-//     k_beta       Jameson sensor (when on; 1-D runs only)            (Mod_Fluxes.f90:366-389)
-//     k_conn       connection-face fluxes by their owner records      (Mod_BC_Fluxes.f90:151-170)
-//     k_bound      boundary cells, records summed in face order        (Mod_BC_Fluxes.f90:105-144)
-//     k_stage3     (k_stage in 1-D runs) interior face fluxes of a tile in shared memory, gathered
-//                  per cell in the odd-then-even order (Mod_Fluxes.f90:421-521), fused with the
-//                  source of a family without evaporation (Mod_Sources.f90:465-622), the residual
+//     k_beta       Jameson sensor (when on)                           (Mod_Fluxes.f90:366-389)
+//     k_flux       the fluxes of the boundary records (Mod_BC_Fluxes.f90:105-170) and of the interior faces
+//                  (Mod_Fluxes.f90:599-685)
+//     k_cells      the cells' update: a cell's boundary faces, then its interior faces in the odd-then-even
+//                  order (Mod_Fluxes.f90:421-521), the source (in the FP32-flux form evaluated here for a family
+//                  without evaporation: Mod_Sources.f90:465-622), the residual
 //                  with the coupler's imports (Lib_Residual.f90:147-210) and the RK update with
 //                  cons<->prim and the state checks (Lib_Newstate.f90:198-219)
 //     (k_irs, k_update when implicit residual smoothing is on: Lib_IRS.f90:34-86)
@@ -42,7 +43,7 @@
 #include <queue>
 #include <functional>
 #include "ice_kernels.cuh"
-#include "ice_stage3.cuh"
+#include "ice_sweep.cuh"
 #include "ice_mlp.cuh"
 #include "ice_tune.h"
 #include "../../include/ice_gpu.h"
@@ -76,17 +77,17 @@ struct FamHost {
   DevBuf<double> S[3];
   DevBuf<unsigned char> inj;
   DevBuf<double> dt, tau, beta;
-  DevBuf<int> bmap;
-  DevBuf<double> Rb, connF, resid, resid2, resid3, src;
+  DevBuf<float> betaf;                       // the FP32-flux form's Jameson weights
+  DevBuf<double> connF, resid, resid2, resid3, src;
   DevBuf<DRec> recs;
   DevBuf<DRec> grecs;                        // the same records ordered for the ghost kernel (upload_recs)
   bool ghost_split = false;                  // the ghost layers in two launches (upload_recs)
-  DevBuf<int> bfirst, blist, own;
-  DevBuf<int> bperm;                         // the boundary cells in the boundary kernel's thread order
-  DevBuf<CUtensorMap> maps[3];               // per state buffer, per block: the staged kernel's TMA maps
-  DevBuf<Tile> tiles3;                       // the staged kernel's tiles
-  int ntile3 = 0;
-  std::vector<Tile> shape3;                  // per block: the staged kernel's tile shape (w, h, bx, by)
+  DevBuf<int> frec;                          // the records whose flux is computed, in the record kernel's thread order
+  int nfrec = 0;
+  DevBuf<ZeroFace> zface;                    // FamDev::zface
+  int nzface = 0;
+  DevBuf<SweepJob> fjobs;                    // the flux kernel's CTAs (ice_sweep.cuh)
+  int nfjob = 0;
   // the evaporation surrogate (FP32-flux form): the network's BF16 image, its standardisation and
   // envelope, its FP32 parameters; on = the stage's source comes from the surrogate source kernel
   DevBuf<unsigned char> mlp_img;
@@ -119,6 +120,11 @@ struct ice_gpu_ctx {
   DevBuf<float4> facef[3];  // the FP32-flux form's geometry (Geo::ff, dlf), rounded from the FP64 arrays
   DevBuf<float> dlf;
   DevBuf<float> gasf;       // the FP32-flux form's copy of the gas (Geo::gasf)
+  // the face fluxes of one family's stage (the families step one after the other), words of 4 or 8 bytes; zeroed
+  // when they are allocated and after a new boundary table (flux_ok)
+  DevBuf<unsigned char> flux[3];
+  int flux_word = 0;
+  bool flux_ok = false;
   bool geo32_ok = false;
   bool have_gas = false;
   std::vector<bool> have_block;
@@ -131,7 +137,6 @@ struct ice_gpu_ctx {
   std::vector<HRec> recs;
   DevBuf<Tile> tiles;
   int ntile = 0, TX = 0, TY = 0, KZ = 0;
-  bool staged = false;    // 2-D and 3-D runs: the staged stage kernel (ice_stage3.cuh)
   DevBuf<NormChunk> chunks;
   DevBuf<double> npart;
   int nchunk = 0;
@@ -229,6 +234,11 @@ static void free_graphs(ice_gpu_ctx* c) {
 // The surrogate source runs for family p: on, trained, a coupled run in the FP32-flux form.
 static bool sur_active(const ice_gpu_ctx* c, int p);
 
+// The stage runs in FP64: the plain form, and every IRS run.
+static bool sweeps64(const ice_gpu_ctx* c) { return c->P.precision != ICE_PREC_FP32FLUX || c->P.irs; }
+// The FP32-flux form's 1-D stage kernel runs (ice_kernels.cuh).
+static bool plane(const ice_gpu_ctx* c) { return !sweeps64(c) && c->P.ndir == 1; }
+
 // The buffer stage srk reads as its stencil (U_{k-1}) when the step starts from buffer `phase`.
 static int stencil_buffer(const ice_gpu_ctx*, int srk, int phase) {
   return srk == 1 ? phase : srk == 2 ? (phase + 1) % 3 : (phase + 2) % 3;
@@ -256,14 +266,15 @@ static FamDev make_famdev(ice_gpu_ctx* c, int p, int srk, int phase) {
   F.inj = H.inj.p;
   F.beta = c->P.shock_detector ? H.beta.p : nullptr;
   F.betaw = H.beta.p;
+  F.betaR = plane(c) || sweeps64(c) ? (void*)H.beta.p : (void*)H.betaf.p;
   F.dt = c->P.time_accurate ? nullptr : H.dt.p;
   F.dtg = &c->st.p->dtglobal;
   F.tau = H.tau.p;
   F.S = H.src.p;
   F.Sf = c->P.precision == ICE_PREC_FP32FLUX ? (float*)H.src.p : nullptr;
-  F.bmap = H.bmap.p;
-  F.Rb = H.Rb.p; F.Rbw = H.Rb.p;
-  F.connF = H.connF.p;
+  F.connF = c->owned.empty() ? nullptr : H.connF.p;
+  for (int d = 0; d < 3; ++d) F.Ff[d] = c->flux[d].p;
+  F.zface = H.zface.p; F.nzface = H.nzface;
   F.cdon = H.cdon.p; F.cw = H.cw.p;
   F.imports = H.have_imp ? H.imp.p : nullptr;
   F.xstep = (c->exchange && c->P.coupled) ? H.xstep.p : nullptr;
@@ -272,7 +283,7 @@ static FamDev make_famdev(ice_gpu_ctx* c, int p, int srk, int phase) {
   static const double RKC[3][3] = {{1.0, 0.0, 0.0}, {1.0, 0.50, 0.0}, {1.0, 0.25, 2.0/3.0}};
   F.rk = RKC[c->P.nrk - 1][srk - 1];
   F.write_tau = srk == c->P.nrk;
-  F.src_ready = (sur_active(c, p) || (c->staged && c->P.coupled && pf.evap != 0)) ? 1 : 0;
+  F.src_ready = (sur_active(c, p) || (c->P.coupled && pf.evap != 0)) ? 1 : 0;
   return F;
 }
 
@@ -440,11 +451,10 @@ static void launch_family(ice_gpu_ctx* c, int p, int srk, int phase, cudaStream_
   a.G = make_geo(c);
   a.F = make_famdev(c, p, srk, phase);
   a.recs = H.recs.p; a.nrec = H.nrec; a.grecs = H.grecs.p; a.ghost_split = H.ghost_split;
-  a.own = H.own.p; a.nown = H.nown;
-  a.bfirst = H.bfirst.p; a.blist = H.blist.p; a.nbc = H.nbc; a.bperm = H.bperm.p;
+  a.frec = H.frec.p; a.nfrec = H.nfrec;
+  a.fjobs = H.fjobs.p; a.nfjob = H.nfjob;
   a.tiles = c->tiles.p; a.ntile = c->ntile; a.TX = c->TX; a.TY = c->TY; a.KZ = c->KZ;
-  a.tiles3 = H.tiles3.p; a.ntile3 = H.ntile3;
-  a.maps = H.maps[stencil_buffer(c, srk, phase)].p;
+  a.plane = plane(c);
   a.mlp_img = sur_active(c, p) ? H.mlp_img.p : nullptr;
   a.mlp_norm = &H.mlp_norm;
   a.ndir = c->P.ndir; a.sd = c->P.shock_detector; a.irs = c->P.irs; a.precision = c->P.precision;
@@ -555,8 +565,9 @@ static long long launches_per_step(const ice_gpu_ctx* c) {
   for (int p = 0; p < c->P.nfam; ++p) n += c->fam[p].have_imp ? 3 : 0;
   for (int p = 0; p < c->P.nfam; ++p) {
     const FamHost& H = c->fam[p];
-    long long per = (H.nrec > 0 ? (H.ghost_split ? 2 : 1) : 0) + (c->P.shock_detector && !c->staged ? 1 : 0) + (H.nown > 0) + (H.nbc > 0) +
-                    (c->P.coupled && (!c->staged || sur_active(c, p) || c->P.fam[p].evap != 0) ? 1 : 0);
+    const bool own_source = c->P.coupled && (sweeps64(c) || plane(c) || sur_active(c, p) || c->P.fam[p].evap != 0);
+    long long per = (H.nrec > 0 ? (H.ghost_split ? 2 : 1) : 0) + (c->P.shock_detector ? 1 : 0) + (own_source ? 1 : 0) +
+                    (H.nfrec + H.nzface > 0 || (!plane(c) && H.nfjob > 0));
     per += c->P.irs ? (2 + 2 * c->P.ndir) : 1;
     n += per * c->P.nrk;
   }
@@ -564,162 +575,136 @@ static long long launches_per_step(const ice_gpu_ctx* c) {
 }
 
 // ---------------------------------------------------------------- set-up helpers
-// The stage kernel's tiles: TX x TY columns of a block (x faces of TX - 1 cells and y faces of
-// TY - 1 cells per tile, the last column and row being the next tile's), KZ planes per tile.
-static void tile_shape(int ndir, int& TX, int& TY, int& KZ) {
-  if (ndir == 1) { TX = 256; TY = 1; KZ = 1; }
-  else if (ndir == 2) { TX = 32; TY = 8; KZ = 1; }
-  else { TX = 16; TY = 16; KZ = 32; }
-  if (const char* e = getenv("ICE_GPU_TILE")) {        // "TXxTYxKZ", for the tile tuner
-    int a, b, k;
-    if (sscanf(e, "%dx%dx%d", &a, &b, &k) == 3 && a * b == 256 && a >= 2 && k >= 1) { TX = a; TY = b; KZ = k; }
-  }
-}
+// The tiles of the FP32-flux form's 1-D stage kernel: TX cells of a row, the last being the next tile's first.
+static void tile_shape(int& TX, int& TY, int& KZ) { TX = 256; TY = 1; KZ = 1; }
 
-// The staged kernel's limits for a closure (Shape<CL> of ice_stage3.cuh).
-static void shape_limits(int closure, int& NT, int& MW, int& MH, int& MB, int& FX, int& FY, int& SXC, int& SYC) {
-  if (closure == ICE_CLOSURE_AG) {
-    NT = Shape<AG>::NT; MW = Shape<AG>::MAXW; MH = Shape<AG>::MAXH; MB = Shape<AG>::MAXBOX;
-    FX = Shape<AG>::FX; FY = Shape<AG>::FY; SXC = Shape<AG>::SXC; SYC = Shape<AG>::SYC;
-  } else {
-    NT = Shape<MK>::NT; MW = Shape<MK>::MAXW; MH = Shape<MK>::MAXH; MB = Shape<MK>::MAXBOX;
-    FX = Shape<MK>::FX; FY = Shape<MK>::FY; SXC = Shape<MK>::SXC; SYC = Shape<MK>::SYC;
-  }
-}
-
-// The staged kernel's tile shape of a block of ni x nj columns: of the shapes W x H that fit the
-// closure's limits (W H <= NT threads, the staged box, the face buffers), the one whose tiles, cut
-// evenly from the block (ceil(ni / W) tiles of ceil(ni / nx) columns, likewise rows), take the fewest
-// passes of the CTA per plane over the whole block: the face tasks (x and y faces below the owned
-// cells, the faces above the last column and row) dealt out to the NT threads, then the z face and
-// the update (zpass of the tuned schedule); at most wcap columns; among equals, the fewest tiles.
-// Returns w, h (the even cut) and the box.
 // The schedule of a closure: its row of the tuned table (ice_tune.h), or ICE_GPU_TUNE="kz,zpass,wcap".
 static TuneRow tune_of(int closure) {
   TuneRow r = kTune[std::min(std::max(closure, 1), 3) - 1];
   if (const char* e = getenv("ICE_GPU_TUNE")) {
     int kz, zp, wc;
-    if (sscanf(e, "%d,%d,%d", &kz, &zp, &wc) == 3 && kz >= 1 && kz <= ST_KZ && zp >= 0 && wc >= 1) r = TuneRow{kz, zp, wc};
+    if (sscanf(e, "%d,%d,%d", &kz, &zp, &wc) == 3 && kz >= 1 && kz <= 32 && zp >= 0 && wc >= 1) r = TuneRow{kz, zp, wc};
   }
   return r;
 }
 
-static Tile tile_shape3(int ni, int nj, int closure) {
-  int NT, MW, MH, MB, FX, FY, SXC, SYC;
-  shape_limits(closure, NT, MW, MH, MB, FX, FY, SXC, SYC);
-  (void)MW;
-  const TuneRow tr = tune_of(closure);
-  Tile best{};
-  long long best_cost = -1, best_tiles = 0;
-  const bool ax = ni >= 2, ay = nj >= 2;
-  const int wmax = ax ? std::min(std::min(ni, NT), tr.wcap) : 1;
-  for (int W = 1; W <= wmax; ++W) {
-    if (st_box_x(W) > 256) break;                 // a TMA box is at most 256 elements along each axis
-    const int hmax = std::min(std::min(nj, MH), NT / W);
-    for (int H = 1; H <= hmax; ++H) {
-      if (st_box_x(W) * (H + 4) > MB || H * (W + 1) > FX || (H + 1) * W > FY) break;
-      if (H * (W + 2) > SXC || (H + 2) * W > SYC) break;   // the FP32-flux form's cell slopes
-      const int nx = (ni + W - 1) / W, ny = (nj + H - 1) / H;
-      const int w = (ni + nx - 1) / nx, h = (nj + ny - 1) / ny;
-      const int tasks = (ax ? w * h + h : 0) + (ay ? w * h + w : 0);
-      const long long tiles = (long long)nx * ny;
-      const long long cost = tiles * ((tasks + NT - 1) / NT + tr.zpass);
-      if (best_cost < 0 || cost < best_cost || (cost == best_cost && tiles < best_tiles)) {
-        best_cost = cost; best_tiles = tiles;
-        best = Tile{0, 0, 0, 0, 0, (short)w, (short)h, (short)st_box_x(w), (short)(h + 4)};
-      }
+// The march length of the flux kernel along one direction, over the owned blocks: per candidate length the
+// threads there are, in waves of the GPU's resident threads, times what a thread does (its faces and the
+// extra slope a march starts with, tr.zpass thirds of a face). A run that fills the GPU marches far, a small
+// one takes one face a thread.
+static int choose_march(const ice_gpu_ctx* c, int d, double slots, const TuneRow& tr) {
+  static const int cand[] = {1, 2, 3, 4, 6, 8, 12, 16, 24, 32};
+  int best = 1;
+  double best_t = 0.0;
+  for (int len : cand) {
+    if (len > tr.kz) break;
+    double thr = 0.0, longest = 0.0;
+    for (int b = 0; b < c->nb; ++b) {
+      if (!c->owned.empty() && !c->owned[b]) continue;
+      const int* n = &c->dims[3 * b];
+      const int m = n[d], nch = (m + len - 1) / len;
+      thr += (double)n[0] * n[1] * n[2] / m * nch;
+      longest = std::max(longest, (double)((m + nch - 1) / nch));
     }
+    const double t = std::max(1.0, thr / slots) * (longest + tr.zpass / 3.0);
+    if (best_t == 0.0 || t < 0.99 * best_t) { best = len; best_t = t; }
   }
   return best;
 }
 
-// The chunk height of the staged kernel's tiles for one family: of a few candidates up to the tuned
-// kz planes, the one whose tiles, handed longest first to the least-loaded of the GPU's resident CTA
-// slots (as the block scheduler hands them out), finish soonest; a tile costs its planes plus the
-// three its prologue loads. Small grids get shorter chunks and more tiles, so that the last wave is
-// not left half empty; large ones keep the largest (a change must gain more than 1 %).
-static int choose_kz(const ice_gpu_ctx* c, const FamHost& H, int slots) {
-  static const int cand[] = {ST_KZ, 28, 24, 20, 16, 12, 8, 4};
-  const int kzmax = tune_of(H.closure).kz;
-  int best = 0;
-  double best_t = 0.0;
-  for (int kz : cand) {
-    if (kz > kzmax) continue;
-    std::vector<int> cost;
+// The flux kernel's CTAs (ice_sweep.cuh) over the owned blocks, by slabs of wcap planes: the x, y and z faces of
+// a slab one after the other, so that the second and third read the state from L2.
+static int build_sweeps(ice_gpu_ctx* c) {
+  int nsm = 148, dev = 0;
+  CK(cudaGetDevice(&dev));
+  CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  const bool f64 = c->P.precision != ICE_PREC_FP32FLUX;
+  for (int p = 0; p < c->P.nfam; ++p) {
+    FamHost& H = c->fam[p];
+    const TuneRow tr = tune_of(H.closure);
+    const int occ = H.closure == ICE_CLOSURE_AG ? (f64 ? SweepOcc<AG, double>::v : SweepOcc<AG, float>::v)
+                                                : (f64 ? SweepOcc<MK, double>::v : SweepOcc<MK, float>::v);
+    const double slots = (double)nsm * occ * SW_NT;
+    const int cy = choose_march(c, 1, slots, tr), cz = choose_march(c, 2, slots, tr);
+    std::vector<SweepJob> f;
+    std::vector<int> slab;           // per job, its slab of the block
     for (int b = 0; b < c->nb; ++b) {
-      int ni = c->dims[3 * b], nj = c->dims[3 * b + 1], nk = c->dims[3 * b + 2];
-      const Tile& sp = H.shape3[b];
-      long long ncol = (long long)((ni + sp.w - 1) / sp.w) * ((nj + sp.h - 1) / sp.h);
-      int nch = (nk + kz - 1) / kz, base = nk / nch, extra = nk % nch;
-      for (int ch = 0; ch < nch; ++ch)
-        for (long long q = 0; q < ncol; ++q) cost.push_back(base + (ch < extra ? 1 : 0) + 3);
+      if (!c->owned.empty() && !c->owned[b]) continue;       // a split run steps its own blocks
+      const int ni = c->dims[3 * b], nj = c->dims[3 * b + 1], nk = c->dims[3 * b + 2];
+      const long long ncell = (long long)ni * nj * nk;
+      auto put = [&](int kind, long long base, int c0, int n, int k) {
+        f.push_back(SweepJob{b, kind, (int)base, c0, n});
+        slab.push_back(k / tr.wcap);
+      };
+      if (ni >= 2)
+        for (long long q = 0; q < ncell; q += SW_XC) put(SW_X, q, 0, 0, (int)(q / ((long long)ni * nj)));
+      auto chunks = [&](int kind, int n, int len, long long cols) {
+        const int nch = (n + len - 1) / len, base = n / nch, extra = n % nch;
+        for (long long q = 0; q < cols; q += SW_NT)
+          for (int ch = 0, k = 0; ch < nch; ++ch) {
+            const int hz = base + (ch < extra ? 1 : 0);
+            put(kind, q, k, hz, kind == SW_Y ? (int)(q / ni) : k);
+            k += hz;
+          }
+      };
+      if (nj >= 2) chunks(SW_Y, nj - 1, cy, (long long)ni * nk);
+      if (nk >= 2) chunks(SW_Z, nk - 1, cz, (long long)ni * nj);
     }
-    std::sort(cost.begin(), cost.end(), std::greater<int>());
-    std::priority_queue<long long, std::vector<long long>, std::greater<long long>> load;
-    for (int q = 0; q < slots; ++q) load.push(0);
-    long long span = 0;
-    for (int x : cost) {
-      long long l = load.top() + x;
-      load.pop(); load.push(l);
-      span = std::max(span, l);
-    }
-    if (best == 0 || (double)span < 0.99 * best_t) { best = kz; best_t = (double)span; }
+    std::vector<int> ord(f.size());
+    for (size_t q = 0; q < ord.size(); ++q) ord[q] = (int)q;
+    std::stable_sort(ord.begin(), ord.end(), [&](int x, int y) {
+      if (f[x].b != f[y].b) return f[x].b < f[y].b;
+      return slab[x] < slab[y];
+    });
+    std::vector<SweepJob> g(f.size());
+    for (size_t q = 0; q < ord.size(); ++q) g[q] = f[ord[q]];
+    H.nfjob = (int)g.size();
+    CK(H.fjobs.alloc(g.size()));
+    if (!g.empty()) CK(cudaMemcpy(H.fjobs.p, g.data(), g.size() * sizeof(SweepJob), cudaMemcpyHostToDevice));
   }
-  return best;
+  return 0;
+}
+
+// The face fluxes: the largest family's, in the word of the running form; the faces no record gives a flux are
+// zero and stay so. Before the first step, after a change of form, after a new boundary table.
+static int ensure_flux(ice_gpu_ctx* c) {
+  const int word = sweeps64(c) ? 8 : 4;
+  if (c->flux_ok && c->flux_word == word) return 0;
+  size_t nc = 0;
+  for (int p = 0; p < c->P.nfam; ++p) nc = std::max(nc, (size_t)c->fam[p].nc);
+  CK(cudaStreamSynchronize(c->stream));
+  if (c->flux_word != word) free_graphs(c);      // they hold the pointers and the form
+  for (int d = 0; d < 3; ++d) {
+    if (c->flux_word != word) CK(c->flux[d].alloc(nc * c->NF[d] * word));
+    CK(cudaMemsetAsync(c->flux[d].p, 0, nc * c->NF[d] * word, c->stream));
+  }
+  for (int p = 0; p < c->P.nfam; ++p)
+    if (word == 4 && c->P.shock_detector && !c->fam[p].betaf.p) {
+      CK(c->fam[p].betaf.alloc(c->NI));
+      free_graphs(c);
+    }
+  c->flux_word = word;
+  c->flux_ok = true;
+  return 0;
 }
 
 static int build_tiles(ice_gpu_ctx* c) {
-  tile_shape(c->P.ndir, c->TX, c->TY, c->KZ);
+  tile_shape(c->TX, c->TY, c->KZ);
   std::vector<Tile> t;
   if (c->P.ndir == 1) {
     for (int b = 0; b < c->nb; ++b) {
       if (!c->owned.empty() && !c->owned[b]) continue;       // a split run steps its own blocks
       int ni = c->dims[3 * b], nj = c->dims[3 * b + 1], nk = c->dims[3 * b + 2];
-      int sx = ni >= 2 ? c->TX - 1 : 1, sy = nj >= 2 ? std::max(c->TY - 1, 1) : 1;
-      for (int k = 0; k < nk; k += c->KZ)
-        for (int j = 0; j < nj; j += sy)
-          for (int i = 0; i < ni; i += sx) t.push_back(Tile{b, i, j, k, std::min(c->KZ, nk - k)});
+      int sx = ni >= 2 ? c->TX - 1 : 1;
+      for (int k = 0; k < nk; ++k)
+        for (int j = 0; j < nj; ++j)
+          for (int i = 0; i < ni; i += sx) t.push_back(Tile{b, i, j, k, 1});
     }
     c->ntile = (int)t.size();
     CK(c->tiles.alloc(t.size()));
     CK(cudaMemcpy(c->tiles.p, t.data(), t.size() * sizeof(Tile), cudaMemcpyHostToDevice));
-  } else {
-    // the staged kernel: column tiles of each block's shape (tile_shape3), each block's height cut
-    // into equal chunks of at most kz planes (choose_kz); the longest first
-    c->staged = true;
-    int nsm = 148;
-    {
-      int dev = 0;
-      CK(cudaGetDevice(&dev));
-      CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    }
-    const int slots = nsm * (c->P.precision == ICE_PREC_FP32FLUX ? 2 : 1);   // the kernel's launch bounds
-    for (int p = 0; p < c->P.nfam; ++p) {
-      FamHost& H = c->fam[p];
-      t.clear();
-      H.shape3.resize(c->nb);
-      for (int b = 0; b < c->nb; ++b) H.shape3[b] = tile_shape3(c->dims[3 * b], c->dims[3 * b + 1], H.closure);
-      const int kz = choose_kz(c, H, slots);
-      for (int b = 0; b < c->nb; ++b) {
-        if (!c->owned.empty() && !c->owned[b]) continue;     // a split run steps its own blocks
-        int ni = c->dims[3 * b], nj = c->dims[3 * b + 1], nk = c->dims[3 * b + 2];
-        const Tile& sp = H.shape3[b];
-        int nch = (nk + kz - 1) / kz, base = nk / nch, extra = nk % nch;
-        for (int ch = 0, k = 0; ch < nch; ++ch) {
-          int hz = base + (ch < extra ? 1 : 0);
-          for (int j = 0; j < nj; j += sp.h)
-            for (int i = 0; i < ni; i += sp.w)
-              t.push_back(Tile{b, i, j, k, hz, (short)std::min((int)sp.w, ni - i), (short)std::min((int)sp.h, nj - j),
-                               sp.bx, sp.by});
-          k += hz;
-        }
-      }
-      std::stable_sort(t.begin(), t.end(), [](const Tile& x, const Tile& y) { return x.nkz > y.nkz; });
-      H.ntile3 = (int)t.size();
-      CK(H.tiles3.alloc(t.size()));
-      CK(cudaMemcpy(H.tiles3.p, t.data(), t.size() * sizeof(Tile), cudaMemcpyHostToDevice));
-    }
   }
+  if (int rc = build_sweeps(c)) return rc;
   // norm chunks: 2048 cells of one block each
   std::vector<NormChunk> ch;
   c->chunk_block.clear();
@@ -734,52 +719,6 @@ static int build_tiles(ice_gpu_ctx* c) {
   CK(c->chunks.alloc(ch.size()));
   CK(cudaMemcpy(c->chunks.p, ch.data(), ch.size() * sizeof(NormChunk), cudaMemcpyHostToDevice));
   CK(c->npart.alloc((size_t)c->nchunk * 5));
-  return 0;
-}
-
-// The staged stage kernel's TMA maps: per family, state buffer and block, a 4-D view (x, y, z,
-// variable) of the block's ghost-cell pool, strides row px, plane pxy and variable NG (all multiples
-// of 16 bytes by the padding of the layout), box bx x by x 1 x nc of the block's tile shape.
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-static EncodeTiledFn encode_tiled() {
-  static EncodeTiledFn fn = nullptr;
-  if (!fn) {
-    void* f = nullptr;
-    cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = (EncodeTiledFn)f;
-  }
-  return fn;
-}
-
-static int build_maps(ice_gpu_ctx* c) {
-  if (!c->staged) return 0;
-  EncodeTiledFn enc = encode_tiled();
-  if (!enc) return fail(c, ICE_GPU_ECUDA, "cuTensorMapEncodeTiled is not available from the driver");
-  std::vector<CUtensorMap> h(c->nb);
-  for (int p = 0; p < c->P.nfam; ++p) {
-    FamHost& H = c->fam[p];
-    for (int buf = 0; buf < 3; ++buf) {
-      for (int b = 0; b < c->nb; ++b) {
-        const DBlock& B = c->hblk[b];
-        cuuint64_t dims[4] = {(cuuint64_t)B.px, (cuuint64_t)(B.nj + 4), (cuuint64_t)(B.nk + 4), (cuuint64_t)H.nc};
-        cuuint64_t strides[3] = {(cuuint64_t)B.px * 8, (cuuint64_t)B.pxy * 8, (cuuint64_t)c->NG * 8};
-        cuuint32_t box[4] = {(cuuint32_t)H.shape3[b].bx, (cuuint32_t)H.shape3[b].by, 1, (cuuint32_t)H.nc};
-        cuuint32_t es[4] = {1, 1, 1, 1};
-        CUresult r = enc(&h[b], CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, (void*)(H.S[buf].p + B.goff), dims, strides, box,
-                         es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (r != CUDA_SUCCESS) return fail(c, ICE_GPU_ECUDA, "cuTensorMapEncodeTiled: error %d (family %d, block %d)",
-                                           (int)r, p + 1, b + 1);
-      }
-      CK(H.maps[buf].alloc(c->nb));
-      CK(cudaMemcpy(H.maps[buf].p, h.data(), c->nb * sizeof(CUtensorMap), cudaMemcpyHostToDevice));
-    }
-  }
   return 0;
 }
 
@@ -853,7 +792,6 @@ int ice_gpu_create(const ice_gpu_params* P, int32_t nblocks, const int32_t* dims
     CKC(H.beta.alloc(I));
     std::vector<double> one(I, 1.0);
     CKC(cudaMemcpy(H.beta.p, one.data(), I * sizeof(double), cudaMemcpyHostToDevice));
-    CKC(H.bmap.alloc(I)); CKC(cudaMemset(H.bmap.p, 0xFF, I * sizeof(int)));
     if (P->coupled) CKC(H.src.alloc((size_t)H.nc * I));
     if (P->irs) { CKC(H.resid.alloc((size_t)H.nc * I)); CKC(H.resid2.alloc((size_t)H.nc * I)); CKC(H.resid3.alloc((size_t)H.nc * I)); }
   }
@@ -863,7 +801,6 @@ int ice_gpu_create(const ice_gpu_params* P, int32_t nblocks, const int32_t* dims
   CKC(cudaEventCreate(&c->ev0)); CKC(cudaEventCreate(&c->ev1));
 #undef CKC
   if (build_tiles(c)) { g_create_err = c->err; return ICE_GPU_ECUDA; }
-  if (build_maps(c)) { g_create_err = c->err; return ICE_GPU_ECUDA; }
   *out = u.release();
   return 0;
 }
@@ -1032,6 +969,7 @@ int ice_gpu_update_params(ice_gpu_ctx* c, const ice_gpu_params* P) {
   CK(cudaStreamSynchronize(c->stream));
   c->P = *P;
   for (int p = 0; p < c->P.nfam; ++p) c->fam[p].riemann = P->fam[p].riemann;
+  c->flux_ok = false;                  // the form or the sensor may have changed
   free_graphs(c);
   return 0;
 }
@@ -1142,14 +1080,13 @@ int ice_gpu_set_records(ice_gpu_ctx* c, int32_t nrec, const int32_t* ri, const d
       d.ca = cos(r.alpha); d.sa = sin(r.alpha); d.cb = cos(r.beta); d.sb = sin(r.beta);
       d.vol_p = 4.0/3.0*kPi*pow(r.radius, 3.0);
       d.cd0 = d.cn1 = d.cn2 = 0;
+      d.next = -1;
     }
     H.nrec = (int)grp.size();
     H.h_grp = grp;
     H.h_recs = dr;
-    if (int rc = upload_recs(c, H)) return rc;
     // boundary cells: block by block in cell order, the records of a cell by face (stable)
     H.h_first.clear(); H.h_list.clear();
-    std::vector<int> bmap(c->NI, -1);
     for (int b = 0; b < c->nb; ++b) {
       const DBlock& B = c->hblk[b];
       long long ncell = (long long)B.ni * B.nj * B.nk;
@@ -1163,7 +1100,6 @@ int ice_gpu_set_records(ice_gpu_ctx* c, int32_t nrec, const int32_t* ri, const d
       }
       for (long long q = 0; q < ncell; ++q) {
         if (head[q] < 0) continue;
-        bmap[B.ioff + q] = (int)H.h_first.size();
         int s0 = (int)H.h_list.size();
         H.h_first.push_back(s0);
         for (int n = head[q]; n >= 0; n = next[n]) H.h_list.push_back(n);
@@ -1176,29 +1112,6 @@ int ice_gpu_set_records(ice_gpu_ctx* c, int32_t nrec, const int32_t* ri, const d
     }
     H.nbc = (int)H.h_first.size();
     H.h_first.push_back((int)H.h_list.size());
-    std::vector<int> dlist(H.h_list.size());
-    for (size_t q = 0; q < H.h_list.size(); ++q) dlist[q] = pos[H.h_list[q]];
-    CK(H.bfirst.alloc(H.h_first.size()));
-    CK(cudaMemcpy(H.bfirst.p, H.h_first.data(), H.h_first.size() * sizeof(int), cudaMemcpyHostToDevice));
-    CK(H.blist.alloc(std::max<size_t>(dlist.size(), 1)));
-    if (!dlist.empty()) CK(cudaMemcpy(H.blist.p, dlist.data(), dlist.size() * sizeof(int), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(H.bmap.p, bmap.data(), c->NI * sizeof(int), cudaMemcpyHostToDevice));
-    CK(H.Rb.alloc((size_t)std::max(H.nbc, 1) * H.nc));
-    // the boundary kernel's thread order: the cells grouped by block, by the face of their first record
-    // and by whether it is a connection, in cell order within a group, so that the threads of a warp take
-    // the same branches (each cell's sum and its slot of Rb are the same in any order)
-    {
-      std::vector<int> perm(H.nbc);
-      for (int q = 0; q < H.nbc; ++q) perm[q] = q;
-      auto key = [&](int q) {
-        const HRec& r = c->recs[H.h_list[H.h_first[q]]];
-        const int conn = (r.type == 101 || r.type == 201) ? 1 : 0;
-        return ((long long)r.b * 8 + r.f) * 2 + conn;
-      };
-      std::stable_sort(perm.begin(), perm.end(), [&](int x, int y) { return key(x) < key(y); });
-      CK(H.bperm.alloc(std::max<size_t>(perm.size(), 1)));
-      if (!perm.empty()) CK(cudaMemcpy(H.bperm.p, perm.data(), perm.size() * sizeof(int), cudaMemcpyHostToDevice));
-    }
     // connection owners, table order
     H.h_own.clear();
     for (int n : grp) {
@@ -1207,12 +1120,71 @@ int ice_gpu_set_records(ice_gpu_ctx* c, int32_t nrec, const int32_t* ri, const d
     }
     H.nown = (int)H.h_own.size();
     H.ncf = ncf;
-    std::vector<int> down(H.h_own.size());
-    for (size_t q = 0; q < H.h_own.size(); ++q) down[q] = pos[H.h_own[q]];
-    CK(H.own.alloc(std::max<size_t>(down.size(), 1)));
-    if (!down.empty()) CK(cudaMemcpy(H.own.p, down.data(), down.size() * sizeof(int), cudaMemcpyHostToDevice));
+    // the records whose flux is computed: connections by their owner; the symmetry records (200) of an MK family
+    // carry none (Mod_BC_Fluxes.f90:128). A face listed twice: its later records follow the first (DRec::next).
+    auto has_flux = [&](const DRec& d) { return d.type != 0 && !(d.type == 200 && H.closure == ICE_CLOSURE_MK); };
+    std::vector<int> fr;
+    for (size_t q = 0; q + 1 < H.h_first.size(); ++q) {
+      int last = -1;
+      for (int l = H.h_first[q]; l < H.h_first[q + 1]; ++l) {
+        const int x = pos[H.h_list[l]];
+        DRec& d = H.h_recs[x];
+        const bool conn = d.type == 101 || d.type == 201;
+        if (!has_flux(d)) continue;
+        if (last >= 0 && !conn && H.h_recs[last].f == d.f) H.h_recs[last].next = x;
+        else if (!conn || d.owner) fr.push_back(x);
+        last = conn ? -1 : x;
+      }
+    }
+    // the record kernel's thread order: by block, face and whether it is a connection, then by cell, so that
+    // the threads of a warp take the same branches and neighbouring cells
+    std::stable_sort(fr.begin(), fr.end(), [&](int x, int y) {
+      const DRec& a = H.h_recs[x]; const DRec& b = H.h_recs[y];
+      if (a.b != b.b) return a.b < b.b;
+      if (a.f != b.f) return a.f < b.f;
+      const int ca = a.type == 101 || a.type == 201, cb = b.type == 101 || b.type == 201;
+      if (ca != cb) return ca < cb;
+      if (a.k != b.k) return a.k < b.k;
+      if (a.j != b.j) return a.j < b.j;
+      return a.i < b.i;
+    });
+    H.nfrec = (int)fr.size();
+    CK(H.frec.alloc(std::max<size_t>(fr.size(), 1)));
+    if (!fr.empty()) CK(cudaMemcpy(H.frec.p, fr.data(), fr.size() * sizeof(int), cudaMemcpyHostToDevice));
     CK(H.connF.alloc((size_t)std::max(ncf, 1) * H.nc));
+    if (int rc = upload_recs(c, H)) return rc;
   }
+  // the boundary faces that a family leaves without a flux where another has one: its record kernel zeroes them
+  if (c->P.nfam > 1) {
+    std::vector<std::vector<long long>> has(c->P.nfam);      // (place of the face) * 4 + direction
+    auto place = [&](const DRec& d) {
+      const DBlock& B = c->hblk[d.b];
+      const int dir = (d.f - 1) / 2;
+      const long long i = d.i + (dir == 0 && d.f % 2 == 0), j = d.j + (dir == 1 && d.f % 2 == 0),
+                      k = d.k + (dir == 2 && d.f % 2 == 0);
+      const long long ni = B.ni + (dir == 0), nj = B.nj + (dir == 1);
+      return (B.foff[dir] + (k * nj + j) * ni + i) * 4 + dir;
+    };
+    std::vector<long long> all;
+    for (int p = 0; p < c->P.nfam; ++p) {
+      for (const DRec& d : c->fam[p].h_recs)
+        if (d.type != 0 && !(d.type == 200 && c->fam[p].closure == ICE_CLOSURE_MK)) has[p].push_back(place(d));
+      std::sort(has[p].begin(), has[p].end());
+      all.insert(all.end(), has[p].begin(), has[p].end());
+    }
+    std::sort(all.begin(), all.end());
+    all.erase(std::unique(all.begin(), all.end()), all.end());
+    for (int p = 0; p < c->P.nfam; ++p) {
+      std::vector<ZeroFace> z;
+      for (long long x : all)
+        if (!std::binary_search(has[p].begin(), has[p].end(), x)) z.push_back(ZeroFace{x / 4, (int)(x % 4)});
+      FamHost& H = c->fam[p];
+      H.nzface = (int)z.size();
+      CK(H.zface.alloc(z.size()));
+      if (!z.empty()) CK(cudaMemcpy(H.zface.p, z.data(), z.size() * sizeof(ZeroFace), cudaMemcpyHostToDevice));
+    }
+  }
+  c->flux_ok = false;                  // the new table's faces without a flux are zeroed again
   c->nchim = 0;
   for (const HRec& r : c->recs) c->nchim += r.type == 102;
   c->have_chimera = c->nchim == 0;
@@ -1372,6 +1344,7 @@ int ice_gpu_step(ice_gpu_ctx* c, int32_t nsteps, ice_gpu_step_out* out) {
   if (!c) return ICE_GPU_EINVAL;
   if (int rc = check_ready(c)) return rc;
   if (int rc = build_geo32(c)) return rc;
+  if (int rc = ensure_flux(c)) return rc;
   if (nsteps < 0) return fail(c, ICE_GPU_EINVAL, "step: nsteps %d", nsteps);
   cudaStream_t s = c->stream;
   if (c->profiling) {
@@ -1466,6 +1439,7 @@ int ice_gpu_step_host(ice_gpu_ctx* c, int32_t nsteps, const double* const* prim_
   if (!c) return ICE_GPU_EINVAL;
   if (int rc = check_ready(c)) return rc;
   if (int rc = build_geo32(c)) return rc;
+  if (int rc = ensure_flux(c)) return rc;
   if (nsteps < 1) return fail(c, ICE_GPU_EINVAL, "step_host: nsteps %d", nsteps);
   if (!prim_in || !prim_out) return fail(c, ICE_GPU_EINVAL, "step_host: null array list");
   if (!c->owned.empty()) return fail(c, ICE_GPU_EINVAL, "step_host: a split run steps through ice_gpu_step");

@@ -1,6 +1,7 @@
 // ice_kernels.cuh -- the kernels of the solve stage that depend on the closure (and the Riemann
-// solver): per-cell dt, the ghost fill of both layers, connection and boundary fluxes, the fused
-// stage kernel and the separate update of the IRS path. Included by the per-closure units
+// solver), but for the flux and cell kernels (ice_sweep.cuh): per-cell dt, the ghost fill of both layers, the
+// boundary records' fluxes, the source, the FP32-flux form's 1-D stage kernel and the separate update of the
+// IRS path. Included by the per-closure units
 // (ice_fam_*.cu) and by ice_gpu.cu, each instantiating what it launches.
 #pragma once
 #include "ice_layout.cuh"
@@ -9,25 +10,14 @@ namespace ice {
 namespace {
 
 // ------------------------------------------------------------------ stencil functor
-struct GStencil {            // q(s, v): cell s = 0..3 of the stencil, variable v
-  const double* P; long long NG, g0, st;
-  __device__ __forceinline__ double operator()(int s, int v) const { return __ldg(P + (long long)v * NG + g0 + s * st); }
-};
-
-template <typename R> struct CStencil {        // converted to R (FP32-flux form)
-  const double* P; long long NG, g0, st;
-  __device__ __forceinline__ R operator()(int s, int v) const { return (R)__ldg(P + (long long)v * NG + g0 + s * st); }
-};
-
-template <typename R, int NC_> struct RegStencil {   // the four cells held in registers (FP32 form)
+template <typename R, int NC_> struct RegStencil {   // q(s, v): cell s = 0..3 of the stencil, variable v
   R v[4][NC_];
   __device__ __forceinline__ R operator()(int s, int q) const { return v[s][q]; }
 };
 
 // One interior face along d between the 0-based cells (i,j,k) and its upper neighbour:
 // face_flux + compute_flux_ (Mod_Fluxes.f90:599-685). Returns true on an unphysical
-// first-order face. The plain form reads the stencil through L1 as the reconstruction needs it;
-// the FP32 form converts it once into registers.
+// first-order face. The stencil is converted once into registers.
 template <int CL, int RS, int LIM, typename R>
 __device__ __forceinline__ bool face_flux(const Geo& G, const FamDev& F, const DBlock& B, int d, int i, int j, int k,
                                          R* flux) {
@@ -49,17 +39,12 @@ __device__ __forceinline__ bool face_flux(const Geo& G, const FamDev& F, const D
   R dll = (R)0.5*l1, dlr = (R)0.5*l2;
   R pl[nc], pr[nc], fl[nc];
   bool bad;
-  if constexpr (sizeof(R) == 8) {
-    CStencil<R> q{F.Up, G.NG, g0, st};
-    bad = reconstruct<CL, LIM, R>(F.limiter, q, dl0, dl1, dl2, dll, dlr, pl, pr, bf);
-  } else {
-    RegStencil<R, nc> q;
+  RegStencil<R, nc> q;
 #pragma unroll
-    for (int s2 = 0; s2 < 4; ++s2)
+  for (int s2 = 0; s2 < 4; ++s2)
 #pragma unroll
-      for (int v = 0; v < nc; ++v) q.v[s2][v] = (R)__ldg(F.Up + (long long)v * G.NG + g0 + s2 * st);
-    bad = reconstruct<CL, LIM, R>(F.limiter, q, dl0, dl1, dl2, dll, dlr, pl, pr, bf);
-  }
+    for (int v = 0; v < nc; ++v) q.v[s2][v] = (R)__ldg(F.Up + (long long)v * G.NG + g0 + s2 * st);
+  bad = reconstruct<CL, LIM, R>(F.limiter, q, dl0, dl1, dl2, dll, dlr, pl, pr, bf);
   const long long fi = fidx(B, d, i, j, k, c + 1);
   const long long NF = G.NF[d];
   const double* fc = G.face[d];
@@ -638,7 +623,7 @@ __global__ void k_ghost(Geo G, FamDev F, const DRec* recs, int nrec, int layers)
 
 // ------------------------------------------------------------------ boundary fluxes
 // A split run's BETA exchange: the Jameson weight of each listed cell (0-based block, i, j, k), as the
-// connection kernel of the same precision and translation unit evaluates it (k_conn).
+// record kernel of the same precision and translation unit evaluates it (rec_face).
 template <typename R>
 __global__ void k_pack_beta(Geo G, FamDev F, const int4* __restrict__ e, int n, double* __restrict__ out) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
@@ -647,53 +632,108 @@ __global__ void k_pack_beta(Geo G, FamDev F, const int4* __restrict__ e, int n, 
   out[q] = F.sd ? (double)beta_cell<R>(F, G.blk[x.x], x.y, x.z, x.w) : 1.0;
 }
 
-template <int CL, int RS, int LIM, typename R>
-__global__ void __launch_bounds__(128, 4) k_conn(Geo G, FamDev F, const DRec* recs, const int* own, int nown, Status* st) {
-  int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= nown) return;
+// The place of the face f of the 0-based cell (i, j, k) in its direction's flux array.
+__device__ __forceinline__ long long face_place(const DBlock& B, int f, int i, int j, int k) {
+  const int d = (f - 1) / 2, c = d == 0 ? i : d == 1 ? j : k;
+  return fidx(B, d, i, j, k, f % 2 == 1 ? c : c + 1);
+}
+
+// The flux x into a cell through its face f, stored as the cells' update reads it: added from the face below
+// the cell, taken off from the face above it.
+template <int CL, typename R>
+__device__ __forceinline__ void put_flux(const Geo& G, const FamDev& F, const DBlock& B, int f, int i, int j, int k,
+                                         const double* x, double sign) {
   constexpr int nc = NC<CL>::v;
-  const DRec& r = recs[own[n]];
-  if (!stepped(G, r.b)) return;
-  R bo = (R)1, bq = (R)1;
-  if (F.sd) {
-    bo = beta_cell<R>(F, G.blk[r.b], r.i, r.j, r.k);
-    // a partner in a block another rank steps: its weight, which that rank sent (ICE_GPU_HALO_BETA)
-    bq = stepped(G, r.pb) ? beta_cell<R>(F, G.blk[r.pb], r.pi, r.pj, r.pk)
-                          : (R)F.beta[iidx(G.blk[r.pb], r.pi, r.pj, r.pk)];
-  }
-  const double bf = (double)mn(bo, bq);
-  double fl[nc];
-  if (record_flux<CL, RS, LIM, R>(G, F, r, fl, &bf)) atomicOr(&st->flags, (unsigned)ICE_GPU_ST_BAD_RECON);
+  const int d = (f - 1) / 2;
+  R* out = (R*)F.Ff[d] + face_place(B, f, i, j, k);
+  const double s = f % 2 == 1 ? sign : -sign;
 #pragma unroll
-  for (int v = 0; v < nc; ++v) F.connF[(long long)r.cf * nc + v] = fl[v];
+  for (int v = 0; v < nc; ++v) out[(long long)v * G.NF[d]] = (R)(s * x[v]);
+}
+
+// The flux through one boundary record's face (Mod_BC_Fluxes.f90:105-170); a connection's is computed by the
+// owner, with the smaller of the two cells' Jameson weights, for both cells.
+template <int CL, int RS, int LIM, typename R>
+__device__ __forceinline__ bool rec_face(const Geo& G, const FamDev& F, const DRec* recs, int rec) {
+  constexpr int nc = NC<CL>::v;
+  const DRec& r = recs[rec];
+  if (!stepped(G, r.b)) return false;
+  double fl[nc];
+  double bf = 0.0;
+  const bool conn = r.type == 101 || r.type == 201;
+  if (conn) {
+    R bo = (R)1, bq = (R)1;
+    if (F.sd) {
+      bo = beta_cell<R>(F, G.blk[r.b], r.i, r.j, r.k);
+      // a partner in a block another rank steps: its weight, which that rank sent (ICE_GPU_HALO_BETA)
+      bq = stepped(G, r.pb) ? beta_cell<R>(F, G.blk[r.pb], r.pi, r.pj, r.pk)
+                            : (R)F.beta[iidx(G.blk[r.pb], r.pi, r.pj, r.pk)];
+    }
+    bf = (double)mn(bo, bq);
+  }
+  bool bad = record_flux<CL, RS, LIM, R>(G, F, r, fl, conn ? &bf : nullptr);
+  for (int n = r.next; n >= 0; n = recs[n].next) {      // a table that lists a face twice: the sum
+    double more[nc];
+    bad |= record_flux<CL, RS, LIM, R>(G, F, recs[n], more, nullptr);
+#pragma unroll
+    for (int v = 0; v < nc; ++v) fl[v] = fl[v] + more[v];
+  }
+  put_flux<CL, R>(G, F, G.blk[r.b], r.f, r.i, r.j, r.k, fl, 1.0);
+  if (conn) {
+    put_flux<CL, R>(G, F, G.blk[r.pb], r.fs, r.pi, r.pj, r.pk, fl, -1.0);
+    if (F.connF) {
+#pragma unroll
+      for (int v = 0; v < nc; ++v) F.connF[(long long)r.cf * nc + v] = fl[v];
+    }
+  }
+  return bad;
+}
+
+// Thread n of the records' fluxes: record frec[n], or after them the faces that only another family's records
+// give a flux (FamDev::zface).
+template <int CL, int RS, int LIM, typename R>
+__device__ __forceinline__ bool rec_thread(const Geo& G, const FamDev& F, const DRec* recs, const int* frec, int nfrec, int n) {
+  if (n < nfrec) return rec_face<CL, RS, LIM, R>(G, F, recs, frec[n]);
+  if (n - nfrec < F.nzface) {
+    const ZeroFace z = F.zface[n - nfrec];
+#pragma unroll
+    for (int v = 0; v < NC<CL>::v; ++v) ((R*)F.Ff[z.d])[(long long)v * G.NF[z.d] + z.at] = (R)0;
+  }
+  return false;
+}
+
+// A split run: the fluxes of the connections whose owner another rank steps, as that rank sent them
+// (ICE_GPU_HALO_FLUX).
+template <int CL, typename R>
+__global__ void k_conn_in(Geo G, FamDev F, const DRec* recs, int nrec) {
+  const int n = blockIdx.x * blockDim.x + threadIdx.x;
+  if (n >= nrec) return;
+  const DRec& r = recs[n];
+  if ((r.type != 101 && r.type != 201) || r.owner || !stepped(G, r.b) || stepped(G, r.pb)) return;
+  put_flux<CL, R>(G, F, G.blk[r.b], r.f, r.i, r.j, r.k, F.connF + (long long)r.cf * NC<CL>::v, -1.0);
 }
 
 template <int CL, int RS, int LIM, typename R>
-__global__ void __launch_bounds__(128, 4) k_bound(Geo G, FamDev F, const DRec* recs, const int* first, const int* list,
-                                                  const int* perm, int nbc, Status* st) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nbc) return;
-  const int c = perm[t];
-  if (!stepped(G, recs[list[first[c]]].b)) return;
-  constexpr int nc = NC<CL>::v;
-  double acc[nc];
+__global__ void __launch_bounds__(128, 4) k_rec(Geo G, FamDev F, const DRec* recs, const int* frec, int nfrec, Status* st) {
+  if (rec_thread<CL, RS, LIM, R>(G, F, recs, frec, nfrec, blockIdx.x * blockDim.x + threadIdx.x))
+    atomicOr(&st->flags, (unsigned)ICE_GPU_ST_BAD_RECON);
+}
+
+// The sum of a cell's boundary fluxes in face order: lo(d, v), hi(d, v) the fluxes of the faces below and above
+// it along d.
+template <int nc, typename LoFn, typename HiFn>
+__device__ __forceinline__ void edge_sum(const DBlock& B, int i, int j, int k, double* acc, const LoFn& lo, const HiFn& hi) {
 #pragma unroll
-  for (int v = 0; v < nc; ++v) acc[v] = 0.0;
-  for (int rr = first[c]; rr < first[c + 1]; ++rr) {
-    const DRec& r = recs[list[rr]];
-    double fl[nc];
-    if (r.type == 200 && CL == MK) continue;
-    if (r.type == 101 || r.type == 201) {
-#pragma unroll
-      for (int v = 0; v < nc; ++v) { double x = F.connF[(long long)r.cf * nc + v]; fl[v] = r.owner ? x : -x; }
-    } else {
-      if (record_flux<CL, RS, LIM, R>(G, F, r, fl, nullptr)) atomicOr(&st->flags, (unsigned)ICE_GPU_ST_BAD_RECON);
-    }
-#pragma unroll
-    for (int v = 0; v < nc; ++v) acc[v] = acc[v] + fl[v];
+  for (int v = 0; v < nc; ++v) {
+    double a = 0.0;
+    if (i == 0) a = a + (double)lo(0, v);
+    if (i == B.ni - 1) a = a - (double)hi(0, v);
+    if (j == 0) a = a + (double)lo(1, v);
+    if (j == B.nj - 1) a = a - (double)hi(1, v);
+    if (k == 0) a = a + (double)lo(2, v);
+    if (k == B.nk - 1) a = a - (double)hi(2, v);
+    acc[v] = a;
   }
-#pragma unroll
-  for (int v = 0; v < nc; ++v) F.Rbw[(long long)c * nc + v] = acc[v];
 }
 
 // ------------------------------------------------------------------ the stage
@@ -732,8 +772,9 @@ __global__ void __launch_bounds__(256, 4) k_source(Geo G, FamDev F) {
   if (F.write_tau) F.tau[q] = (double)tau;
 }
 
-// The stage kernel. One CTA of TX x TY threads (256) owns a column tile of one block and marches
-// up a chunk of KZ planes. On each plane every thread computes exactly one x face (the face below
+// The stage kernel of the FP32-flux form's 1-D runs, whose residual sums and divisions are FP64. One CTA of
+// TX x TY threads (256) owns a column tile of one block and marches up a chunk of KZ planes. On each
+// plane every thread computes exactly one x face (the face below
 // its cell), one y face and one z face (the face above its cell; the one below comes from the
 // plane before, or is computed once at the chunk's first plane) into shared memory, so the work is
 // the same for every thread; then each cell of the tile's (TX-1) x (TY-1) interior takes its two
@@ -793,10 +834,12 @@ k_stage(Geo G, FamDev F, const Tile* tiles, int TX, int TY, int KZ, int write_r,
     __syncthreads();
     if (owner) {
       const long long q = iidx(B, i, j, k);
-      const int bc = F.bmap[q];
       double r[nc];
-#pragma unroll
-      for (int v = 0; v < nc; ++v) r[v] = bc >= 0 ? F.Rb[(long long)bc * nc + v] : 0.0;
+      edge_sum<nc>(B, i, j, k, r, [&](int d, int v) {
+        return ((const R*)F.Ff[d])[(long long)v * G.NF[d] + fidx(B, d, i, j, k, d == 0 ? i : d == 1 ? j : k)];
+      }, [&](int d, int v) {
+        return ((const R*)F.Ff[d])[(long long)v * G.NF[d] + fidx(B, d, i, j, k, (d == 0 ? i : d == 1 ? j : k) + 1)];
+      });
       // direction 1: face tid+1 is the cell's upper face, face tid its lower one
       if (ax) {
         const int ci = i + 1, n = B.ni;
@@ -943,15 +986,15 @@ __global__ void k_time(Status* st, int time_accurate) {
 
 
 // ------------------------------------------------------------------ sensor
-__global__ void k_beta(Geo G, FamDev F) {
+template <typename R> __global__ void k_beta(Geo G, FamDev F) {
   long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= G.NI) return;
   const DBlock& B = G.blk[find_block(G.blk, G.nb, q)];
   int i, j, k; decode(B, q, i, j, k);
   const double* P = F.Up;   // variable 0: density
-  F.betaw[q] = sd_rho<double>(P[gidx(B, i, j, k)], P[gidx(B, i - 1, j, k)], P[gidx(B, i + 1, j, k)],
-                      P[gidx(B, i, j - 1, k)], P[gidx(B, i, j + 1, k)],
-                      P[gidx(B, i, j, k - 1)], P[gidx(B, i, j, k + 1)]);
+  ((R*)F.betaR)[q] = sd_rho<R>((R)P[gidx(B, i, j, k)], (R)P[gidx(B, i - 1, j, k)], (R)P[gidx(B, i + 1, j, k)],
+                      (R)P[gidx(B, i, j - 1, k)], (R)P[gidx(B, i, j + 1, k)],
+                      (R)P[gidx(B, i, j, k - 1)], (R)P[gidx(B, i, j, k + 1)]);
 }
 
 

@@ -1,7 +1,6 @@
 // ice_layout.cuh -- the device layout of the solve stage: blocks, geometry, records, status,
 // the per-family view the kernels read, and the launch interface of the per-closure units.
 #pragma once
-#include <cuda.h>
 #include <cuda_runtime.h>
 #include "ice_physics.cuh"
 
@@ -12,7 +11,7 @@ namespace ice {
 struct DBlock {
   int ni, nj, nk;
   int px;             // row pitch of the ghost-cell pools: ni + 4 rounded up to even, so that every row,
-                      // plane and block starts on a 16-byte boundary (the TMA tensor maps need it)
+                      // plane and block starts on a 16-byte boundary
   long long pxy;      // plane pitch, px * (nj + 4)
   long long goff;     // ghost-cell pools (1-gc:n+gc)^3
   long long ioff;     // interior pools
@@ -44,6 +43,7 @@ struct DRec {                // one boundary record, 0-based cells
   int b, i, j, k, f, type;
   int bs, is, js, ks, fs;
   int owner, cf;             // cf 0-based (-1 when none)
+  int next;                  // another record of the same cell and face (place in the family's records), or -1
   int pb, pi, pj, pk;        // the partner's cell (connections)
   int normal_dir;
   double massflux, velocity, alpha, beta, temperature, radius, gfixed;
@@ -87,6 +87,8 @@ __device__ __forceinline__ long long gstride(const DBlock& B, int d) {
   return d == 0 ? 1LL : d == 1 ? (long long)B.px : B.pxy;
 }
 
+struct ZeroFace { long long at; int d; };    // a face: its place in direction d's flux array
+
 struct FamDev {              // what the kernels of one family read
   int closure, riemann, nc, limiter, sd, coupled, drag, heat, blow;
   unsigned int frozen_mask;  // bit v: slot v+1 frozen
@@ -98,15 +100,17 @@ struct FamDev {              // what the kernels of one family read
   unsigned char* inj;
   const double* beta;        // NI, or null (1)
   double* betaw;
+  void* betaR;               // NI: the Jameson weights of a stage in the form's precision (ice_sweep.cuh)
   const double* dt;          // NI (steady) or null
   const double* dtg;         // &status->dtglobal (time-accurate)
   double* tau;               // NI
   double* S;                 // [v][NI]: the stage's source (coupled runs)
   float* Sf;                 // the FP32-flux form's source, [v][NI] floats in the same buffer (else null)
-  const int* bmap;           // NI: boundary-cell index or -1
-  const double* Rb;          // [nbcell][nc]
-  double* Rbw;
-  double* connF;             // [ncf][nc]
+  double* connF;             // [ncf][nc]: a split run's connection fluxes on their way to and from other ranks
+  void* Ff[3];               // the face fluxes of a stage [v][NF] per direction, in the form's precision; a face
+                             // of the block's boundary holds its record's flux, zero where no record has one
+  const ZeroFace* zface;     // the boundary faces without a flux that another family's stage gave one
+  int nzface;
   const int4* cdon;          // chimera donors: 0-based block, i, j, k
   const double* cw;          // chimera donor weights
   const double* imports;     // [v][NI]: the coupler's rates into the cells, or null
@@ -127,10 +131,15 @@ struct EmptyScan {
   unsigned int filled, pad;
 };
 
-// A column tile of a block and its chunk of nkz planes. The staged stage kernel's tiles also carry
-// their owned columns and rows (w, h) and the staged box of their block (bx, by: the TMA box's x and y).
-struct Tile { int b, i0, j0, k0, nkz; short w, h, bx, by; };
+// A tile of the 1-D stage kernel.
+struct Tile { int b, i0, j0, k0, nkz; };
 struct MlpNorm;
+
+// One CTA's share of the flux kernel (ice_sweep.cuh): the x faces above the cells base.. of block b (flat over
+// the block), or the y or z faces above the cells c0 .. c0 + n - 1 of the columns base.. (flat over the plane
+// across them).
+enum { SW_X = 0, SW_Y = 1, SW_Z = 2 };
+struct SweepJob { int b, kind, base, c0, n; };
 struct NormChunk { int b; long long q0, q1; };
 
 // Everything one family's stage needs, for the launcher of its closure's translation unit.
@@ -140,15 +149,13 @@ struct LaunchArgs {
   const DRec* recs; int nrec;
   const DRec* grecs;                                 // the records in the ghost kernel's order
   int ghost_split;                                   // a record's second layer reads another's first
-  const int* own; int nown;
-  const int* bfirst; const int* blist; int nbc;
-  const int* bperm;                                  // the boundary cells in the boundary kernel's thread order
+  const int* frec; int nfrec;                        // the records whose flux is computed, in thread order
+  const SweepJob* fjobs; int nfjob;                  // the flux kernel's CTAs
   const Tile* tiles; int ntile; int TX, TY, KZ;     // the 1-D stage kernel's tiles
-  const Tile* tiles3; int ntile3;                    // the staged stage kernel's tiles (2-D and 3-D runs)
-  const CUtensorMap* maps;                           // per block: the TMA map of U_{k-1} (the stencil buffer)
   const unsigned char* mlp_img;                      // the family's surrogate network (null: the plain closure)
   const MlpNorm* mlp_norm;
   int ndir, sd, irs, precision;
+  int plane;                                         // the FP32-flux form's 1-D stage kernel runs (ice_kernels.cuh)
   double irs_beta;
   double* resid; double* resid2; double* resid3;
   Status* st;
@@ -174,12 +181,18 @@ void launch_source_ig_f64(const LaunchArgs& a);
 void launch_source_ig_f32(const LaunchArgs& a);
 void launch_source_ag_f64(const LaunchArgs& a);
 void launch_source_ag_f32(const LaunchArgs& a);
-void launch_bound_mk_f64(const LaunchArgs& a);
-void launch_bound_mk_f32(const LaunchArgs& a);
-void launch_bound_ig_f64(const LaunchArgs& a);
-void launch_bound_ig_f32(const LaunchArgs& a);
-void launch_bound_ag_f64(const LaunchArgs& a);
-void launch_bound_ag_f32(const LaunchArgs& a);
+void launch_flux_mk_f64(const LaunchArgs& a);
+void launch_beta_mk_f64(const LaunchArgs& a);
+void launch_flux_mk_f32(const LaunchArgs& a);
+void launch_beta_mk_f32(const LaunchArgs& a);
+void launch_flux_ig_f64(const LaunchArgs& a);
+void launch_beta_ig_f64(const LaunchArgs& a);
+void launch_flux_ig_f32(const LaunchArgs& a);
+void launch_beta_ig_f32(const LaunchArgs& a);
+void launch_flux_ag_f64(const LaunchArgs& a);
+void launch_beta_ag_f64(const LaunchArgs& a);
+void launch_flux_ag_f32(const LaunchArgs& a);
+void launch_beta_ag_f32(const LaunchArgs& a);
 void launch_pack_beta_mk_f64(const LaunchArgs& a, const int4* e, int n, double* out);
 void launch_pack_beta_mk_f32(const LaunchArgs& a, const int4* e, int n, double* out);
 void launch_pack_beta_ig_f64(const LaunchArgs& a, const int4* e, int n, double* out);

@@ -27,6 +27,7 @@
 #include <cmath>
 #include "../../include/ice_gpu.h"
 #include "../../include/ice_math.h"
+#include "../../include/ice_div.h"
 
 namespace ice {
 
@@ -84,6 +85,16 @@ __device__ __forceinline__ float th(float x) { return tanhf(x); }
 template <typename R> __device__ __forceinline__ R tol_picard() { return sizeof(R) == 8 ? (R)1.e-12 : (R)1.e-5f; }
 template <typename R> __device__ __forceinline__ R tol_newton() { return sizeof(R) == 8 ? (R)1.0e-13 : (R)1.0e-6f; }
 
+// FP64 quotients without a branch each (ice_div.h): `ok` stays true while every operand lies in the range
+// where they are the IEEE quotients; where it does not, the caller evaluates the same expressions with `/`.
+__device__ __forceinline__ bool dividend(double a) {
+  return ice_div_in(a) || ((ice_div_hi(a) | (unsigned)__double2loint(a)) == 0u);
+}
+__device__ __forceinline__ double quot(double a, double b, bool& ok) {
+  ok = ok && ice_div_by(b) && dividend(a);
+  return ice_div_quot(a, b, ice_div_recip(b));
+}
+
 // Limiters the kernels specialise at compile time; any other runs through the run-time switch.
 constexpr int LIM_ANY = -1;
 
@@ -126,8 +137,31 @@ template <int CL, typename R> __device__ __forceinline__ void prim2cons(const R*
   }
 }
 
+// The FP32-flux form's FP64 prim -> cons with its fused multiply-adds written out: which product of a sum is
+// fused decides the last bit, and IG's pressure is what a cancellation leaves of it, so the choice is not the
+// compiler's.
+template <int CL> __device__ __forceinline__ void prim2cons_fma(const double* p, double* c, double cp) {
+  if constexpr (CL == AG) {
+    prim2cons<CL, double>(p, c, cp);
+  } else {
+    const double n2 = __fma_rn(p[3], p[3], __fma_rn(p[1], p[1], __dmul_rn(p[2], p[2])));
+    const double m = __dmul_rn(p[0], cp);
+    c[0] = p[0];
+    c[1] = p[0]*p[1]; c[2] = p[0]*p[2]; c[3] = p[0]*p[3];
+    if constexpr (CL == MK) {
+      c[4] = __fma_rn(m, p[4], __dmul_rn(__dmul_rn(0.5, p[0]), n2));
+      c[5] = p[5];
+    } else {
+      c[4] = __fma_rn(p[0], n2, __dmul_rn(3.0, p[4]));
+      c[5] = __fma_rn(0.5, c[4], __dmul_rn(m, p[5]));
+      c[6] = p[6];
+    }
+  }
+}
+
 // cons -> prim with the reference's floors (Lib_Model_*: cons_2_prim_*). FAST (the FP32-flux form):
-// the velocities multiply by one reciprocal of the density instead of three divisions.
+// the velocities multiply by one reciprocal of the density instead of three divisions, and the fused
+// multiply-adds of the speed are written out, as in prim2cons_fma.
 template <int CL, bool FAST = false> __device__ __forceinline__ void cons2prim(const double* c, double* p, double cp) {
   const double eps = epsv<double>();
   p[0] = c[0];
@@ -137,7 +171,9 @@ template <int CL, bool FAST = false> __device__ __forceinline__ void cons2prim(c
   } else {
     p[1] = c[1] / (p[0] + eps); p[2] = c[2] / (p[0] + eps); p[3] = c[3] / (p[0] + eps);
   }
-  double n2 = p[1]*p[1] + p[2]*p[2] + p[3]*p[3];
+  double n2;
+  if constexpr (FAST) n2 = __fma_rn(p[3], p[3], __fma_rn(p[2], p[2], __dmul_rn(p[1], p[1])));
+  else n2 = p[1]*p[1] + p[2]*p[2] + p[3]*p[3];
   if constexpr (CL == MK) {
     p[4] = (c[4] - 0.5*p[0]*n2) / (cp*p[0] + eps);
     p[5] = c[5];
@@ -387,6 +423,98 @@ template <int LIM, typename R> __device__ __forceinline__ R limiter(int lim, R x
   return phi * x;
 }
 
+// The general forms, out of line: the operands ice_div.h does not take.
+static __device__ __noinline__ double quot_any(double a, double b) { return a / b; }
+static __device__ __noinline__ double limiter_any(int lim, double x, double y, double cx, double cy) {
+  return limiter<LIM_ANY, double>(lim, x, y, cx, cy);
+}
+
+// A difference quotient whose limiter takes the branchless quotients: zero, or 2^-98 <= |s| < 2^200. The range
+// keeps the operands that formed it normal too, and s + 1e-30 away from cancellation.
+__device__ __forceinline__ bool slope_in(double s) {
+  const unsigned h = ice_div_hi(s);
+  return h - (925u << 20) < (298u << 20) || (h | (unsigned)__double2loint(s)) == 0u;
+}
+
+// The difference quotients (b - a) / dl of every variable; false when the limiter has to take the general
+// quotients for one of them (FP64; slope_in).
+template <int nc, typename R> __device__ __forceinline__ bool quotients(const R* a, const R* b, R dl, R* s) {
+  if constexpr (sizeof(R) == 4) {
+    const R i = rcp_fast(dl);
+#pragma unroll
+    for (int v = 0; v < nc; ++v) s[v] = (b[v] - a[v]) * i;
+    return true;
+  } else {
+    // one reciprocal for every variable; the chains of the variables run side by side
+    const R y = ice_div_recip(dl);
+    bool ok = ice_div_by(dl);
+#pragma unroll
+    for (int v = 0; v < nc; ++v) {
+      s[v] = ice_div_quot(b[v] - a[v], dl, y);
+      ok = ok && slope_in(s[v]);
+    }
+    if (!ok) {
+#pragma unroll
+      for (int v = 0; v < nc; ++v) s[v] = quot_any(b[v] - a[v], dl);
+    }
+    return ok;
+  }
+}
+
+// The limited slopes of every variable from their two difference quotients: limiter(x, y) of each (0 for a
+// first-order cell). In FP64 the slope ratios of all variables are formed side by side, then the limiter's
+// formula, its run-time choice made once; fast: every quotient passed slope_in.
+template <int nc, int LIM, typename R>
+__device__ __forceinline__ void limited(int lim, const R* x, const R* y, R cx, R cy, bool first, bool fast, R* s) {
+  if constexpr (sizeof(R) == 4) {
+#pragma unroll
+    for (int v = 0; v < nc; ++v) s[v] = first ? (R)0 : limiter<LIM>(lim, x[v], y[v], cx, cy);
+  } else {
+    const int kind = LIM == LIM_ANY ? lim : LIM;
+    R ru[nc], phi[nc];
+    unsigned low = 0;                // the largest low word of a divisor (all ones: ice_div_by)
+#pragma unroll
+    for (int v = 0; v < nc; ++v) {
+      const R d = x[v] + (R)1e-30;
+      low = max(low, (unsigned)__double2loint(d));
+      ru[v] = ice_div_quot(y[v], d, ice_div_recip(d));
+    }
+#define ICE_EACH(expr) { _Pragma("unroll") for (int v = 0; v < nc; ++v) { const R r = ru[v]; phi[v] = (expr); } }
+    switch (kind) {
+      case ICE_LIM_MINMOD: ICE_EACH(mx((R)0, mn((R)1, r))) break;
+      case ICE_LIM_VANLEER: {
+#pragma unroll
+        for (int v = 0; v < nc; ++v) {           // phi is 0 for r <= 0, and so is what the bounds make of it
+          ru[v] = ru[v] > (R)0 ? ru[v] : (R)0;
+          const R d = (R)1 + ru[v];
+          low = max(low, (unsigned)__double2loint(d));
+          phi[v] = ice_div_quot(ru[v] + ru[v], d, ice_div_recip(d));
+        }
+        break;
+      }
+      case ICE_LIM_VANALBADA: ICE_EACH(quot_any(r*r + r, r*r + (R)1)) break;
+      case ICE_LIM_OSPRE: ICE_EACH(quot_any((R)1.5*(r*r + r), r*r + r + (R)1)) break;
+      case ICE_LIM_UMIST: ICE_EACH(mx((R)0, mn(mn(mn((R)2*r, (R)0.25 + (R)0.75*r), (R)0.75 + (R)0.25*r), (R)2))) break;
+      case ICE_LIM_OSHER: ICE_EACH(mx((R)0, mn(r, (R)1.5))) break;
+      case ICE_LIM_SWEBY: ICE_EACH(mx(mx((R)0, mn((R)1.5*r, (R)1)), mn(r, (R)1.5))) break;
+      case ICE_LIM_MC: ICE_EACH(mx((R)0, mn(mn((R)2*r, (R)0.5*((R)1 + r)), (R)2))) break;
+      case ICE_LIM_KOREN: ICE_EACH(mx((R)0, mn((R)2*r, mn(quot_any((R)1 + (R)2*r, (R)3), (R)2)))) break;
+      case ICE_LIM_SUPERBEE: ICE_EACH(mx(mx((R)0, mn((R)2*r, (R)1)), mn(r, (R)2))) break;
+      default: first = true;        // first order
+    }
+#undef ICE_EACH
+#pragma unroll
+    for (int v = 0; v < nc; ++v) {
+      if (LIM == ICE_LIM_VANLEER || (kind != ICE_LIM_MINMOD && ru[v] > (R)0)) phi[v] = mn(mn(phi[v], cx), cy*ru[v]);
+      s[v] = first ? (R)0 : phi[v] * x[v];
+    }
+    if ((!fast || low == 0xffffffffu) && !first) {
+#pragma unroll
+      for (int v = 0; v < nc; ++v) s[v] = limiter_any(kind, x[v], y[v], cx, cy);
+    }
+  }
+}
+
 // The four cells of a stencil: a source of values q(s, v), s = 0..3 (prev, local, next, next2).
 // state_reconstruction + slope_bounds; returns true when the first-order fallback is itself
 // unphysical (report_stencil).
@@ -410,27 +538,30 @@ __device__ __forceinline__ bool reconstruct(int lim, const Q& q, R dl0, R dl1, R
     for (int v = 0; v < nc; ++v) pr[v] = q(2, v);
   }
   bool st_l = first_l, st_r = first_r;
-  // FP32-flux form: the three lengths' reciprocals once per face in place of a division per variable
-  R i0 = (R)1, i1 = (R)1, i2 = (R)1;
-  if constexpr (sizeof(R) == 4) { i0 = rcp_fast(dl0); i1 = rcp_fast(dl1); i2 = rcp_fast(dl2); }
+  // the limited slopes, which do not change while the weight halves
+  R sl[nc], sr[nc];
+  {
+    R a[nc], b[nc], s0[nc], s1[nc], s2[nc];
+#pragma unroll
+    for (int v = 0; v < nc; ++v) { a[v] = q(0, v); b[v] = q(1, v); }
+    const bool k0 = quotients<nc, R>(a, b, dl0, s0);
+#pragma unroll
+    for (int v = 0; v < nc; ++v) a[v] = q(2, v);
+    const bool k1 = quotients<nc, R>(b, a, dl1, s1);
+#pragma unroll
+    for (int v = 0; v < nc; ++v) b[v] = q(3, v);
+    const bool k2 = quotients<nc, R>(a, b, dl2, s2);
+    limited<nc, LIM, R>(lim, s1, s0, cxl, cyl, first_l, k0 && k1, sl);
+    limited<nc, LIM, R>(lim, s2, s1, cxr, cyr, first_r, k1 && k2, sr);
+  }
   // the weight halves each pass: from any weight <= 1 it is below 1e-18 within 61 passes; the
   // cap only guards a non-finite weight, for which the reference would not end
   for (int pass = 0; (!st_l || !st_r) && pass < 256; ++pass) {
     if (pass == 255) limval = (R)0;
 #pragma unroll
     for (int v = 0; v < nc; ++v) {
-      R a1 = q(1, v), a2 = q(2, v);
-      R slope1 = sizeof(R) == 4 ? (a2 - a1) * i1 : (a2 - a1) / dl1;
-      if (!first_l) {
-        R slope0 = sizeof(R) == 4 ? (a1 - q(0, v)) * i0 : (a1 - q(0, v)) / dl0;
-        R sl = limiter<LIM>(lim, slope1, slope0, cxl, cyl) * limval;
-        pl[v] = a1 + sl*dll;
-      }
-      if (!first_r) {
-        R slope2 = sizeof(R) == 4 ? (q(3, v) - a2) * i2 : (q(3, v) - a2) / dl2;
-        R sr = limiter<LIM>(lim, slope2, slope1, cxr, cyr) * limval;
-        pr[v] = a2 - sr*dlr;
-      }
+      if (!first_l) pl[v] = q(1, v) + (sl[v]*limval)*dll;
+      if (!first_r) pr[v] = q(2, v) - (sr[v]*limval)*dlr;
     }
     if (!first_l) st_l = check_prim<CL>(pl);
     if (!first_r) st_r = check_prim<CL>(pr);
@@ -537,6 +668,32 @@ template <int CL> __device__ __forceinline__ void rusanov_pair(const float* p1, 
   }
 }
 
+// The signal speeds of the two states of a face: wavespeed of each, in FP64 with their quotients side by side.
+template <int CL, typename R> __device__ __forceinline__ void wavespeeds(const R* p1, const R* p4, const R* n, R& s1, R& s4) {
+  if constexpr (sizeof(R) == 4 || CL == MK) {
+    s1 = wavespeed<CL>(p1, n); s4 = wavespeed<CL>(p4, n);
+  } else {
+    R a1, a4;
+    bool ok = true;
+    if constexpr (CL == IG) {
+      const R t = ice_div_recip((R)3);
+      const R b1 = p1[4] + p1[4] + p1[4], b4 = p4[4] + p4[4] + p4[4];
+      ok = dividend(b1) && dividend(b4);
+      a1 = (R)3*ice_div_quot(b1, (R)3, t); a4 = (R)3*ice_div_quot(b4, (R)3, t);
+    } else {
+      const R q1 = n[0]*(p1[4]*n[0] + p1[5]*n[1] + p1[6]*n[2]) + n[1]*(p1[5]*n[0] + p1[7]*n[1] + p1[8]*n[2]) +
+                   n[2]*(p1[6]*n[0] + p1[8]*n[1] + p1[9]*n[2]);
+      const R q4 = n[0]*(p4[4]*n[0] + p4[5]*n[1] + p4[6]*n[2]) + n[1]*(p4[5]*n[0] + p4[7]*n[1] + p4[8]*n[2]) +
+                   n[2]*(p4[6]*n[0] + p4[8]*n[1] + p4[9]*n[2]);
+      a1 = (R)3*fmax(q1, (R)0); a4 = (R)3*fmax(q4, (R)0);
+    }
+    s1 = quot(a1, p1[0] + epsv<R>(), ok);
+    s4 = quot(a4, p4[0] + epsv<R>(), ok);
+    if (ok) { s1 = sqrt(s1); s4 = sqrt(s4); }
+    else { s1 = wavespeed<CL>(p1, n); s4 = wavespeed<CL>(p4, n); }
+  }
+}
+
 template <int CL, typename R> __device__ __forceinline__ void rusanov(const R* p1, const R* p4, const R* n, R* f, R cp) {
   if constexpr (sizeof(R) == 4) {
     rusanov_pair<CL>(p1, p4, n, f, cp);
@@ -546,7 +703,8 @@ template <int CL, typename R> __device__ __forceinline__ void rusanov(const R* p
   R c1[nc], c4[nc], f1[nc], f4[nc];
   R vn1 = p1[1]*n[0] + p1[2]*n[1] + p1[3]*n[2];
   R vn4 = p4[1]*n[0] + p4[2]*n[1] + p4[3]*n[2];
-  R s1 = wavespeed<CL>(p1, n), s4 = wavespeed<CL>(p4, n);
+  R s1, s4;
+  wavespeeds<CL, R>(p1, p4, n, s1, s4);
   prim2cons<CL>(p1, c1, cp); prim2cons<CL>(p4, c4, cp);
   R A = fabs(vn1 - s1);
   A = mx(A, (R)fabs(vn4 - s4)); A = mx(A, (R)fabs(vn1 + s1)); A = mx(A, (R)fabs(vn4 + s4));
@@ -566,7 +724,8 @@ template <int CL, typename R> __device__ __forceinline__ void hlle(const R* p1, 
   constexpr int nc = NC<CL>::v;
   R vn1 = p1[1]*n[0] + p1[2]*n[1] + p1[3]*n[2];
   R vn4 = p4[1]*n[0] + p4[2]*n[1] + p4[3]*n[2];
-  R s1 = wavespeed<CL>(p1, n), s4 = wavespeed<CL>(p4, n);
+  R s1, s4;
+  wavespeeds<CL, R>(p1, p4, n, s1, s4);
   R r1 = sqrt(p1[0]), r4 = sqrt(p4[0]);
   R uR = (r1*p1[1] + r4*p4[1]) / (r1 + r4);
   R vR = (r1*p1[2] + r4*p4[2]) / (r1 + r4);

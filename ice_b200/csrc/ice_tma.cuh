@@ -1,9 +1,7 @@
-// ice_tma.cuh -- the tensor-memory-accelerator (TMA) loads and the shared-memory mbarriers the stage
-// kernel stages its state planes with (sm_90+ PTX, used here on sm_100a). Loads only: no store, no
-// reduce, no cluster multicast. Every wait is bounded: past the bound the caller sets an error flag
-// in the step status instead of spinning on.
+// ice_tma.cuh -- shared-memory mbarriers and the proxy fences of the surrogate's tensor-core kernel (sm_90+ PTX,
+// used here on sm_100a). Every wait is bounded: past the bound the caller sets an error flag in the step
+// status instead of spinning on.
 #pragma once
-#include <cuda.h>
 #include <cuda_runtime.h>
 #include <cstdint>
 
@@ -17,20 +15,15 @@ __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(smem_u32(bar)), "r"(count) : "memory");
 }
 
-// Makes the initialised barrier visible to the async proxy (the TMA unit) before its first use.
+// Makes the initialised barrier visible to the async proxy before its first use.
 __device__ __forceinline__ void fence_mbar_init() {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
 
 // Orders this thread's earlier generic-proxy accesses of shared memory before later async-proxy
-// (TMA) writes to it.
+// accesses to it.
 __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
-               :: "r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
 
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
@@ -58,20 +51,6 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint64
       if (mbar_try_wait(bar, parity)) return true;
     if (global_ns() - t0 > limit_ns) return false;
   }
-}
-
-// One 4-D tiled TMA load (x, y, z, variable) of the box the tensor map defines into shared memory,
-// completing on `bar` with the box's byte count. x * 8 bytes must be a multiple of 16.
-__device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, uint64_t* bar,
-                                            int x, int y, int z, int v) {
-  asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-               " [%0], [%1, {%2, %3, %4, %5}], [%6];"
-               :: "r"(smem_u32(dst)), "l"((uint64_t)map), "r"(x), "r"(y), "r"(z), "r"(v), "r"(smem_u32(bar))
-               : "memory");
-}
-
-__device__ __forceinline__ void prefetch_tmap(const CUtensorMap* map) {
-  asm volatile("prefetch.tensormap [%0];" :: "l"((uint64_t)map) : "memory");
 }
 
 }  // namespace ice

@@ -1,4 +1,4 @@
-"""The tuner of the staged stage kernel's schedule: for each closure it times the kernel on one GPU for
+"""The tuner of the flux kernel's schedule: for each closure it times the stage on one GPU for
 every candidate (kz, zpass, wcap) of ice_b200/csrc/ice_tune.h and writes the fastest into that file,
 with the measurements, for the library's next build.
 
@@ -8,7 +8,7 @@ The workload is the 48-block tree's recipe (seed 9, blocks of U[16, 160] cells p
 first --blocks blocks, one family at a time in the chosen form (FP32 fluxes, FP64 accumulation),
 so that each closure's kernel is timed on the block shapes it meets. A candidate is applied through
 ICE_GPU_TUNE, which the library reads when a context is created; the time is the mean CUDA-event
-duration of the stage kernel's launches over --steps profiled steps after one warm-up step.
+duration of a stage's flux and cell kernels over --steps profiled steps after one warm-up step.
 """
 from __future__ import annotations
 
@@ -30,8 +30,8 @@ from ice_b200.solver import Solver  # noqa: E402
 
 CLOSURES = ("MK", "IG", "AG")
 KZ = (8, 16, 24, 32)
-ZPASS = (1, 2, 3, 4)
-WCAP = {"MK": (16, 32, 64), "IG": (16, 32, 64), "AG": (16, 24, 32)}
+ZPASS = (2, 4, 8)
+WCAP = {"MK": (4, 8, 16), "IG": (4, 8, 16), "AG": (4, 8, 16)}
 KC_STAGE = 4
 
 
@@ -49,19 +49,18 @@ def time_candidate(lib, case, steps: int) -> float:
 
 
 def header(rows: dict, table: dict, what: str) -> str:
-    lines = ["// ice_tune.h -- the staged stage kernel's schedule per closure, as the tuner (ice_b200/tune.py) chose",
-             "// it by timing the kernel on one B200. Rewritten by the tuner; the library reads it at build time.",
+    lines = ["// ice_tune.h -- the flux kernel's schedule per closure (ice_sweep.cuh), as the tuner (ice_b200/tune.py) chose",
+             "// it by timing the stage on one B200. Rewritten by the tuner; the library reads it at build time.",
              "//",
-             "//   kz     the most planes one tile's chunk takes (its height is cut into equal chunks of at most kz,",
-             "//          fewer when that balances the last wave of CTAs better: choose_kz)",
-             "//   zpass  the passes of the CTA per plane that the tile-shape cost adds to the face tasks' passes",
-             "//          (the z face and the update): the larger, the more it favours few, full tiles",
-             "//   wcap   the widest tile, in owned columns",
+             "//   kz     the longest march of a thread along y or z, in faces (shorter where the run is small: choose_march)",
+             "//   zpass  the start of a march (the slope of its first cell), in thirds of a face: the larger, the longer",
+             "//          the marches a small run takes",
+             "//   wcap   the planes of a slab, whose x, y and z faces run one after the other",
              "//",
              "// The environment variable ICE_GPU_TUNE=\"kz,zpass,wcap\" overrides the row of every closure (the",
              "// tuner's sweep uses it).",
              "//",
-             f"// Measured: {what}. Stage-kernel launch in ms, the chosen row first:"]
+             f"// Measured: {what}. Flux and cell kernels of a stage in ms, the chosen row first:"]
     for cl in CLOSURES:
         ranked = sorted(table[cl].items(), key=lambda kv: kv[1])
         lines.append(f"//   {cl}: " + ", ".join(f"{k} {v:.4f}" for k, v in ranked[:6]) +
