@@ -926,7 +926,7 @@ template <typename R> __device__ __forceinline__ void evap_invariants(EvapEnv<R>
 }
 
 // gasSideRate with the five gas-side models (Lib_Evaporation.f90:205-224, 287-521)
-template <typename R> __device__ void gas_side(const EvapEnv<R>& e, R Ys, R BM, R& md, R& Qd, bool& ovr) {
+template <typename R> __device__ __forceinline__ void gas_side(const EvapEnv<R>& e, R Ys, R BM, R& md, R& Qd, bool& ovr) {
   const R pi = (R)kPi;
   md = (R)0; Qd = (R)0; ovr = false;
   const double* ep = e.ep;
@@ -1021,7 +1021,7 @@ template <typename R> __device__ void gas_side(const EvapEnv<R>& e, R Ys, R BM, 
 }
 
 // evaporation + lkCorrection (Lib_Evaporation.f90:145-261)
-template <typename R> __device__ void evaporation(R rhog, R Tg, R gamma, R Rg, R mug, R kg, R Tp, R dp, R Re,
+template <typename R> __device__ __forceinline__ void evaporation(R rhog, R Tg, R gamma, R Rg, R mug, R kg, R Tp, R dp, R Re,
                                                   const Mat& m, R& mdot, R& Qd, bool& ovr) {
   mdot = (R)0; Qd = (R)0; ovr = false;
   if (m.evap == 0) return;
@@ -1153,7 +1153,7 @@ template <typename R> __device__ __forceinline__ void closure_rates(R rhog, R Tg
 
 // compute_source_ + cell_surface on the ITC/clamp, non-burning, constant-property path.
 // gas = rho u v w T. Returns tau. INF when Cd == 0.
-template <int CL, typename R> __device__ R cell_source(const R* p, const R* gas, R gR, R ggam, R gk, R gmu,
+template <int CL, typename R> __device__ __forceinline__ R cell_source(const R* p, const R* gas, R gR, R ggam, R gk, R gmu,
                                                       const Mat& m, int drag_sel, int heat_sel, int blow, R* s) {
   const CellPhys<R> c = cell_phys<CL, R>(p, gas, gR, ggam, gk, gmu, m, drag_sel, heat_sel);
   R mdot, Qconv;
