@@ -55,12 +55,13 @@ void launch_family_t(const LaunchArgs& a) {
     tick(KC_SOURCE);
   }
   if (a.xchg) a.xchg(a, ICE_GPU_HALO_CELLS);   // the remote source cells of the ghost layers
-  if (a.nrec > 0) {
+  if (a.ngrec + a.ncopy > 0) {
+    const unsigned g = grid((long long)a.ngrec + a.ncopy, 128);
     if (a.ghost_split) {
-      k_ghost<CL><<<grid(a.nrec, 128), 128, 0, s>>>(a.G, a.F, a.grecs, a.nrec, 1);
-      k_ghost<CL><<<grid(a.nrec, 128), 128, 0, s>>>(a.G, a.F, a.grecs, a.nrec, 2);
+      k_ghost<CL><<<g, 128, 0, s>>>(a.G, a.F, a.grecs, a.ngrec, 1, nullptr, 0, 0);
+      k_ghost<CL><<<g, 128, 0, s>>>(a.G, a.F, a.grecs, a.ngrec, 2, nullptr, 0, 0);
     } else {
-      k_ghost<CL><<<grid(a.nrec, 128), 128, 0, s>>>(a.G, a.F, a.grecs, a.nrec, 3);
+      k_ghost<CL><<<g, 128, 0, s>>>(a.G, a.F, a.grecs, a.ngrec, 3, a.gcopy, a.ncopy, a.next);
     }
     tick(KC_GHOST);
   }

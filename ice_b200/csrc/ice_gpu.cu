@@ -80,7 +80,9 @@ struct FamHost {
   DevBuf<float> betaf;                       // the FP32-flux form's Jameson weights
   DevBuf<double> connF, resid, resid2, resid3, src;
   DevBuf<DRec> recs;
-  DevBuf<DRec> grecs;                        // the same records ordered for the ghost kernel (upload_recs)
+  DevBuf<DRec> grecs;                        // the ghost kernel's records, and its copies (upload_recs)
+  DevBuf<GhostCopy> gcopy;
+  int ngrec = 0, ncopy = 0, next = 0;
   bool ghost_split = false;                  // the ghost layers in two launches (upload_recs)
   DevBuf<int> frec;                          // the records whose flux is computed, in the record kernel's thread order
   int nfrec = 0;
@@ -122,7 +124,8 @@ struct ice_gpu_ctx {
   DevBuf<float> gasf;       // the FP32-flux form's copy of the gas (Geo::gasf)
   // the face fluxes of one family's stage (the families step one after the other), words of 4 or 8 bytes; zeroed
   // when they are allocated and after a new boundary table (flux_ok)
-  DevBuf<unsigned char> flux[3];
+  DevBuf<unsigned char> flux;
+  size_t flux_at[3] = {0, 0, 0};
   int flux_word = 0;
   bool flux_ok = false;
   bool geo32_ok = false;
@@ -273,7 +276,7 @@ static FamDev make_famdev(ice_gpu_ctx* c, int p, int srk, int phase) {
   F.S = H.src.p;
   F.Sf = c->P.precision == ICE_PREC_FP32FLUX ? (float*)H.src.p : nullptr;
   F.connF = c->owned.empty() ? nullptr : H.connF.p;
-  for (int d = 0; d < 3; ++d) F.Ff[d] = c->flux[d].p;
+  for (int d = 0; d < 3; ++d) F.Ff[d] = c->flux.p + c->flux_at[d];
   F.zface = H.zface.p; F.nzface = H.nzface;
   F.cdon = H.cdon.p; F.cw = H.cw.p;
   F.imports = H.have_imp ? H.imp.p : nullptr;
@@ -450,7 +453,8 @@ static void launch_family(ice_gpu_ctx* c, int p, int srk, int phase, cudaStream_
   LaunchArgs a;
   a.G = make_geo(c);
   a.F = make_famdev(c, p, srk, phase);
-  a.recs = H.recs.p; a.nrec = H.nrec; a.grecs = H.grecs.p; a.ghost_split = H.ghost_split;
+  a.recs = H.recs.p; a.nrec = H.nrec; a.ghost_split = H.ghost_split;
+  a.grecs = H.grecs.p; a.ngrec = H.ngrec; a.gcopy = H.gcopy.p; a.ncopy = H.ncopy; a.next = H.next;
   a.frec = H.frec.p; a.nfrec = H.nfrec;
   a.fjobs = H.fjobs.p; a.nfjob = H.nfjob;
   a.tiles = c->tiles.p; a.ntile = c->ntile; a.TX = c->TX; a.TY = c->TY; a.KZ = c->KZ;
@@ -566,7 +570,7 @@ static long long launches_per_step(const ice_gpu_ctx* c) {
   for (int p = 0; p < c->P.nfam; ++p) {
     const FamHost& H = c->fam[p];
     const bool own_source = c->P.coupled && (sweeps64(c) || plane(c) || sur_active(c, p) || c->P.fam[p].evap != 0);
-    long long per = (H.nrec > 0 ? (H.ghost_split ? 2 : 1) : 0) + (c->P.shock_detector ? 1 : 0) + (own_source ? 1 : 0) +
+    long long per = (H.ngrec + H.ncopy > 0 ? (H.ghost_split ? 2 : 1) : 0) + (c->P.shock_detector ? 1 : 0) + (own_source ? 1 : 0) +
                     (H.nfrec + H.nzface > 0 || (!plane(c) && H.nfjob > 0));
     per += c->P.irs ? (2 + 2 * c->P.ndir) : 1;
     n += per * c->P.nrk;
@@ -674,10 +678,13 @@ static int ensure_flux(ice_gpu_ctx* c) {
   for (int p = 0; p < c->P.nfam; ++p) nc = std::max(nc, (size_t)c->fam[p].nc);
   CK(cudaStreamSynchronize(c->stream));
   if (c->flux_word != word) free_graphs(c);      // they hold the pointers and the form
+  size_t n = 0;
   for (int d = 0; d < 3; ++d) {
-    if (c->flux_word != word) CK(c->flux[d].alloc(nc * c->NF[d] * word));
-    CK(cudaMemsetAsync(c->flux[d].p, 0, nc * c->NF[d] * word, c->stream));
+    c->flux_at[d] = n;
+    n += (nc * c->NF[d] * word + 255) & ~(size_t)255;
   }
+  if (c->flux_word != word) CK(c->flux.alloc(n));
+  CK(cudaMemsetAsync(c->flux.p, 0, n, c->stream));
   for (int p = 0; p < c->P.nfam; ++p)
     if (word == 4 && c->P.shock_detector && !c->fam[p].betaf.p) {
       CK(c->fam[p].betaf.alloc(c->NI));
@@ -974,22 +981,23 @@ int ice_gpu_update_params(ice_gpu_ctx* c, const ice_gpu_params* P) {
   return 0;
 }
 
-// The family's device records (table order, which the boundary and connection kernels index), and a
-// copy for the ghost kernel ordered by block, face and cell with the first index fastest, so that the
-// threads of a warp fill neighbouring ghost cells of one face (a record's ghosts are its own, so the
-// order of the fills does not change a value). ghost_split: some record's block (or, for a connection,
-// its source block) is one cell deep along the record's face direction, so that record's second ghost
-// layer reads the first layer of the opposite face's record; the ghost kernel then runs as two launches.
+// The family's device records (table order, which the record kernel indexes), and what the ghost kernel
+// reads, ordered by block, face and cell with the first index fastest, so that the threads of a warp fill
+// neighbouring ghost cells of one face (a record's ghosts are its own, so the order of the fills does not
+// change a value): the copying records of the stepped blocks as GhostCopy, the others as they are.
+// ghost_split: some record's block (or, for a connection, its source block) is one cell deep along the
+// record's face direction, so that record's second ghost layer reads the first layer of the opposite face's
+// record; the ghost kernel then runs as two launches, every record as it is.
 static int upload_recs(ice_gpu_ctx* c, FamHost& H) {
   const std::vector<DRec>& dr = H.h_recs;
   CK(H.recs.alloc(dr.size()));
-  CK(H.grecs.alloc(dr.size()));
   H.ghost_split = false;
   for (const DRec& r : dr) {
     if (r.type == 0 || r.type == 102) continue;
     if (c->dims[3 * r.b + (r.f - 1) / 2] == 1) H.ghost_split = true;
     if ((r.type == 101 || r.type == 201) && c->dims[3 * r.bs + (r.fs - 1) / 2] == 1) H.ghost_split = true;
   }
+  H.ngrec = H.ncopy = H.next = 0;
   if (dr.empty()) return 0;
   CK(cudaMemcpy(H.recs.p, dr.data(), dr.size() * sizeof(DRec), cudaMemcpyHostToDevice));
   std::vector<int> ord(dr.size());
@@ -1002,9 +1010,37 @@ static int upload_recs(ice_gpu_ctx* c, FamHost& H) {
     if (a.j != b.j) return a.j < b.j;
     return a.i < b.i;
   });
-  std::vector<DRec> g(dr.size());
-  for (size_t q = 0; q < ord.size(); ++q) g[q] = dr[ord[q]];
-  CK(cudaMemcpy(H.grecs.p, g.data(), g.size() * sizeof(DRec), cudaMemcpyHostToDevice));
+  auto at = [&](int b, int i, int j, int k) {
+    const DBlock& B = c->hblk[b];
+    return (unsigned)(B.goff + (k + 2) * B.pxy + (long long)(j + 2) * B.px + (i + 2));
+  };
+  std::vector<DRec> g;
+  std::vector<GhostCopy> ext, copy;
+  for (int q : ord) {
+    const DRec& r = dr[q];
+    const bool conn = r.type == 101 || r.type == 201;
+    if (H.ghost_split || !(conn || r.type == 0 || r.type == 400)) { g.push_back(r); continue; }
+    if (!c->owned.empty() && !c->owned[r.b]) continue;       // a split run fills its own blocks' ghosts
+    const int g0 = (r.f == 1) - (r.f == 2), g1 = (r.f == 3) - (r.f == 4), g2 = (r.f == 5) - (r.f == 6);
+    GhostCopy x;
+    x.g1 = at(r.b, r.i - g0, r.j - g1, r.k - g2);
+    x.g2 = r.type == 0 ? kNoGhost : at(r.b, r.i - 2 * g0, r.j - 2 * g1, r.k - 2 * g2);
+    if (conn) {
+      const int s0 = (r.fs == 1) - (r.fs == 2), s1 = (r.fs == 3) - (r.fs == 4), s2 = (r.fs == 5) - (r.fs == 6);
+      x.m = at(r.bs, r.is, r.js, r.ks); x.p = at(r.bs, r.is + s0, r.js + s1, r.ks + s2);
+    } else {
+      x.m = at(r.b, r.i, r.j, r.k); x.p = at(r.b, r.i + g0, r.j + g1, r.k + g2);
+    }
+    (conn ? copy : ext).push_back(x);
+  }
+  H.next = (int)ext.size();
+  ext.insert(ext.end(), copy.begin(), copy.end());
+  H.ncopy = (int)ext.size();
+  H.ngrec = (int)g.size();
+  CK(H.grecs.alloc(g.size()));
+  CK(H.gcopy.alloc(ext.size()));
+  if (!g.empty()) CK(cudaMemcpy(H.grecs.p, g.data(), g.size() * sizeof(DRec), cudaMemcpyHostToDevice));
+  if (!ext.empty()) CK(cudaMemcpy(H.gcopy.p, ext.data(), ext.size() * sizeof(GhostCopy), cudaMemcpyHostToDevice));
   return 0;
 }
 
@@ -1155,7 +1191,16 @@ int ice_gpu_set_records(ice_gpu_ctx* c, int32_t nrec, const int32_t* ri, const d
     if (int rc = upload_recs(c, H)) return rc;
   }
   // the boundary faces that a family leaves without a flux where another has one: its record kernel zeroes them
-  if (c->P.nfam > 1) {
+  bool alike = true;                   // every family has the same codes face by face, and none an MK family's 200
+  for (int p = 0; p < c->P.nfam && alike; ++p) {
+    const std::vector<DRec>& x = c->fam[p].h_recs; const std::vector<DRec>& y = c->fam[0].h_recs;
+    alike = x.size() == y.size();
+    for (size_t q = 0; q < x.size() && alike; ++q)
+      alike = x[q].type == y[q].type && x[q].b == y[q].b && x[q].f == y[q].f && x[q].i == y[q].i && x[q].j == y[q].j &&
+              x[q].k == y[q].k && x[q].type != 200;
+  }
+  for (int p = 0; p < c->P.nfam; ++p) c->fam[p].nzface = 0;
+  if (!alike) {
     std::vector<std::vector<long long>> has(c->P.nfam);      // (place of the face) * 4 + direction
     auto place = [&](const DRec& d) {
       const DBlock& B = c->hblk[d.b];
@@ -1604,6 +1649,8 @@ int ice_gpu_set_partition(ice_gpu_ctx* c, const int32_t* owned) {
   }
   CK(cudaStreamSynchronize(c->stream));
   free_graphs(c);
+  for (int p = 0; p < c->P.nfam; ++p)
+    if (int rc = upload_recs(c, c->fam[p])) return rc;       // the ghost copies are of the stepped blocks
   if (build_tiles(c)) return ICE_GPU_ECUDA;
   return 0;
 }

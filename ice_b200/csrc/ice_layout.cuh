@@ -55,6 +55,13 @@ struct DRec {                // one boundary record, 0-based cells
   int cd0, cn1, cn2;
 };
 
+// The two ghost cells of a record that copies cells (0, 400, 101, 201), as places in a variable's pool: the first
+// layer g1 takes m, the second g2 takes p (a 400 record 3 g1 - 3 m + p); code 0 has no second (g2 = kNoGhost).
+// Sixteen bytes in place of a record's two hundred. A pool has fewer than 2^32 places: three buffers of six
+// doubles for each are more than the GPU holds.
+struct GhostCopy { unsigned m, p, g1, g2; };
+constexpr unsigned kNoGhost = 0xffffffffu;
+
 struct Status {
   unsigned int flags;
   unsigned int pad;
@@ -147,7 +154,8 @@ struct LaunchArgs {
   Geo G;
   FamDev F;
   const DRec* recs; int nrec;
-  const DRec* grecs;                                 // the records in the ghost kernel's order
+  const GhostCopy* gcopy; int ncopy, next;           // the ghosts that copy cells, the extrapolating ones first
+  const DRec* grecs; int ngrec;                      // the other records, in the ghost kernel's order
   int ghost_split;                                   // a record's second layer reads another's first
   const int* frec; int nfrec;                        // the records whose flux is computed, in thread order
   const SweepJob* fjobs; int nfjob;                  // the flux kernel's CTAs
