@@ -119,6 +119,7 @@ struct ice_gpu_ctx {
   long long NG = 0, NI = 0, NR = 0, NF[3] = {0, 0, 0};
   DevBuf<DBlock> blk;
   DevBuf<double> face[3], vol, dl, M, gas;
+  DevBuf<double> row;       // Geo::row, formed from M with each block's metrics
   DevBuf<float4> facef[3];  // the FP32-flux form's geometry (Geo::ff, dlf), rounded from the FP64 arrays
   DevBuf<float> dlf;
   DevBuf<float> gasf;       // the FP32-flux form's copy of the gas (Geo::gasf)
@@ -295,7 +296,7 @@ static Geo make_geo(ice_gpu_ctx* c) {
   G.blk = c->blk.p; G.nb = c->nb;
   G.NG = c->NG; G.NI = c->NI; G.NR = c->NR;
   for (int d = 0; d < 3; ++d) { G.NF[d] = c->NF[d]; G.face[d] = c->face[d].p; }
-  G.vol = c->vol.p; G.dl = c->dl.p; G.M = c->M.p; G.gas = c->gas.p;
+  G.vol = c->vol.p; G.dl = c->dl.p; G.M = c->M.p; G.gas = c->gas.p; G.row = c->row.p;
   for (int d = 0; d < 3; ++d) G.ff[d] = c->facef[d].p;
   G.dlf = c->dlf.p;
   G.gasf = c->gasf.p;
@@ -782,6 +783,7 @@ int ice_gpu_create(const ice_gpu_params* P, int32_t nblocks, const int32_t* dims
   CKC(c->vol.alloc(I));
   CKC(c->dl.alloc((size_t)3 * R));
   CKC(c->M.alloc((size_t)9 * I));
+  CKC(c->row.alloc((size_t)12 * I));
   if (P->coupled) CKC(c->gas.alloc((size_t)9 * I));
   for (int p = 0; p < P->nfam; ++p) {
     FamHost& H = c->fam[p];
@@ -868,6 +870,9 @@ int ice_gpu_set_block(ice_gpu_ctx* c, int32_t b1, const double* f1, const double
     }
     CK(cudaMemcpy(c->M.p + (long long)comp * c->NI + B.ioff, tmp.data(), ncell * sizeof(double), cudaMemcpyHostToDevice));
   }
+  CK(cudaStreamSynchronize(c->stream));
+  k_rows<<<grid_of(ncell), 256, 0, c->stream>>>(c->M.p, c->row.p, c->NI, B.ioff, ncell);
+  CK(cudaGetLastError());
   c->have_block[b1 - 1] = true;
   c->geo32_ok = false;
   return 0;

@@ -174,7 +174,10 @@ __device__ __forceinline__ void decode(const DBlock& B, long long q, int& i, int
 // cell's metric rows are read once for all families; the cell's indices come from its block by 32-bit
 // arithmetic (ice_gpu_create refuses a block of 2^31 cells or more). Per family the operations of
 // compute_dt_ in its order; the global step is the smallest over every family and cell (an exact
-// minimum, so the order of the families does not matter).
+// minimum, so the order of the families does not matter). Bound by its reads. The rows' unit vectors and
+// moduli are formed once, when the metrics are set (k_rows: the scaled norm and the divisions were two
+// thirds of the kernel's instructions), and the signal speeds' and the rate's quotients are branchless:
+// IG, 128 x 126 x 129 cells: 122 us before, 89 now.
 struct DtFam {
   const double* Up;
   const double* tau;
@@ -187,18 +190,67 @@ struct DtArgs {
   double cfl, dt_max, tau_factor;
 };
 
+// The unit vector and the modulus of every metric row of the cells q0 .. q0 + n - 1, as compute_dt_ forms them.
+__global__ void k_rows(const double* __restrict__ M, double* __restrict__ row, long long NI, long long q0, long long n) {
+  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
+    const long long q = q0 + e;
+    for (int d = 0; d < 3; ++d) {
+      const double t0 = M[(long long)d * NI + q], t1 = M[(long long)(3 + d) * NI + q], t2 = M[(long long)(6 + d) * NI + q];
+      const double g = norm2_3(t0, t1, t2);
+      row[(long long)(4 * d) * NI + q] = t0 / g;
+      row[(long long)(4 * d + 1) * NI + q] = t1 / g;
+      row[(long long)(4 * d + 2) * NI + q] = t2 / g;
+      row[(long long)(4 * d + 3) * NI + q] = g;
+    }
+  }
+}
+
+// The signal speeds of state p along the three rows (wavespeed of each).
+template <int CL>
+__device__ __forceinline__ void row_speeds(const double* p, const double (*vs)[4], double* ws) {
+  if constexpr (CL == MK) {
+    ws[0] = ws[1] = ws[2] = 0.0;
+  } else if constexpr (CL == IG) {
+    ws[0] = ws[1] = ws[2] = wavespeed<CL>(p, vs[0]);         // the same along every row
+  } else {
+    const double b = p[0] + epsv<double>(), y = ice_div_recip(b);
+    bool ok = ice_div_by(b);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {                // (the rows beyond ndir are zero)
+      const double* n = vs[d];
+      const double pnn = n[0]*(p[4]*n[0] + p[5]*n[1] + p[6]*n[2]) +
+                         n[1]*(p[5]*n[0] + p[7]*n[1] + p[8]*n[2]) +
+                         n[2]*(p[6]*n[0] + p[8]*n[1] + p[9]*n[2]);
+      const double a = 3.0*fmax(pnn, 0.0);
+      ok = ok && dividend(a);
+      ws[d] = sqrt(ice_div_quot(a, b, y));
+    }
+    if (!ok) {
+#pragma unroll
+      for (int d = 0; d < 3; ++d) ws[d] = wavespeed<CL>(p, vs[d]);
+    }
+  }
+}
+
 template <int CL>
 __device__ __forceinline__ double family_dt(const Geo& G, const DtFam& f, const DtArgs& a, long long q, long long g,
-                                            const double (*vs)[3], const double* gn, int it) {
-  constexpr int nc = NC<CL>::v;
+                                            const double (*vs)[4], int it) {
+  constexpr int nc = NC<CL>::v, used = CL == MK ? 4 : CL == IG ? 5 : 10;      // what a rate depends on
   double p[nc];
 #pragma unroll
-  for (int v = 0; v < nc; ++v) p[v] = f.Up[(long long)v * G.NG + g];
-  double rate = 0.0;
-  for (int d = 0; d < a.ndir; ++d)
-    rate = rate + (fabs(p[1]*vs[d][0] + p[2]*vs[d][1] + p[3]*vs[d][2]) + wavespeed<CL>(p, vs[d])) * gn[d];
+  for (int v = 0; v < used; ++v) p[v] = f.Up[(long long)v * G.NG + g];
+  double ws[3], rate = 0.0;
+  row_speeds<CL>(p, vs, ws);
+#pragma unroll
+  for (int d = 0; d < 3; ++d)
+    if (d < a.ndir) rate = rate + (fabs(p[1]*vs[d][0] + p[2]*vs[d][1] + p[3]*vs[d][2]) + ws[d]) * vs[d][3];
   double dt = (double)1e+5f;
-  if (rate > 0.0) dt = mn(dt, 1.0/rate);
+  if (rate > 0.0) {
+    bool ok = true;
+    double r = quot(1.0, rate, ok);
+    if (!ok) r = 1.0/rate;
+    dt = mn(dt, r);
+  }
   dt = dt * a.cfl;
   if (it <= a.ramp) dt = dt * (double)it / (double)a.ramp;
   dt = mn(dt, a.dt_max);
@@ -210,7 +262,7 @@ __device__ __forceinline__ double family_dt(const Geo& G, const DtFam& f, const 
   return dt;
 }
 
-__global__ void __launch_bounds__(256, 6) k_dt_all(Geo G, DtArgs a, Status* st) {
+__global__ void __launch_bounds__(256, 4) k_dt_all(Geo G, DtArgs a, Status* st) {
   long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   double dt = INFINITY;
   const int bq = q < G.NI ? find_block(G.blk, G.nb, q) : 0;
@@ -219,18 +271,17 @@ __global__ void __launch_bounds__(256, 6) k_dt_all(Geo G, DtArgs a, Status* st) 
     const unsigned l = (unsigned)(q - B.ioff), ni = (unsigned)B.ni, nj = (unsigned)B.nj;
     const unsigned i = l % ni, jk = l / ni, j = jk % nj, k = jk / nj;
     const long long g = gidx(B, (int)i, (int)j, (int)k);
-    double vs[3][3], gn[3];
-    for (int d = 0; d < a.ndir; ++d) {
-      double t0 = G.M[(long long)d * G.NI + q], t1 = G.M[(long long)(3 + d) * G.NI + q], t2 = G.M[(long long)(6 + d) * G.NI + q];
-      gn[d] = norm2_3(t0, t1, t2);
-      vs[d][0] = t0 / gn[d]; vs[d][1] = t1 / gn[d]; vs[d][2] = t2 / gn[d];
-    }
+    double vs[3][4];
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+#pragma unroll
+      for (int m = 0; m < 4; ++m) vs[d][m] = d < a.ndir ? G.row[(long long)(4 * d + m) * G.NI + q] : 0.0;
     const int it = st->iter;
     for (int p = 0; p < a.nf; ++p) {
       const DtFam& f = a.f[p];
-      double d = f.closure == ICE_CLOSURE_MK ? family_dt<MK>(G, f, a, q, g, vs, gn, it)
-               : f.closure == ICE_CLOSURE_IG ? family_dt<IG>(G, f, a, q, g, vs, gn, it)
-                                             : family_dt<AG>(G, f, a, q, g, vs, gn, it);
+      double d = f.closure == ICE_CLOSURE_MK ? family_dt<MK>(G, f, a, q, g, vs, it)
+               : f.closure == ICE_CLOSURE_IG ? family_dt<IG>(G, f, a, q, g, vs, it)
+                                             : family_dt<AG>(G, f, a, q, g, vs, it);
       dt = mn(dt, d);
     }
   }

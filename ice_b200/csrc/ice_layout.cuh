@@ -27,6 +27,7 @@ struct Geo {                 // geometry shared by the families
   const double* vol;         // NI
   const double* dl;          // 3 SoA components of NR
   const double* M;           // 9 SoA components of NI (column-major c(3,3))
+  const double* row;         // per direction the metric row's unit vector and modulus, 4 SoA components of NI each
   const double* gas;         // 9 SoA components of NI: rho u v w T R gam k mu
   // the FP32-flux form's copies of the face geometry (nx, ny, nz, A of a face in one 16-byte word) and
   // of the cell lengths, rounded once from the FP64 arrays above (null in the plain form)
