@@ -4,10 +4,10 @@
 // One call of ice_gpu_step replaces `call Explicit_Step(grid)` (src/lib/driver/Wrap_Solve.f90:26;
 // numerics/time/explicit/Mod_Explicit.f90:11-245). Every array is resident in HBM; a step is a
 // CUDA graph of:
-//   k_begin        iteration counters, dt reset                      (Mod_Explicit.f90:40-44)
 //   k_dt_all       per-cell CFL dt of every family + global min (FP64)  (Mod_dt.f90:11-112,256-275)
 //   (k_empty_scan, k_empty_apply for a family with the coupler's imports: Mod_dt.f90:134-242)
-//   k_time         dtglobal, time += dt                               (Mod_Explicit.f90:67-73)
+//                  and the end of the dt part: dtglobal, time += dt, counters (Mod_Explicit.f90:40-73; k_time
+//                  where the bounds of imports or of other ranks come after it)
 //   per family, per RK stage:
 //     k_source     the source (plain form; an evaporating family of the FP32-flux form; 1-D runs), or the
 //                  surrogate's k_source_mlp                            (Mod_Sources.f90:465-622)
@@ -508,18 +508,20 @@ static int next_phase(const ice_gpu_ctx* c, int phase) {
 // One Explicit_Step on stream s starting from buffer `phase`: the step's dt over every family, then
 // each family's RK stages (the families are independent of one another within a step).
 static void enqueue_step_dt(ice_gpu_ctx* c, int phase, cudaStream_t s, void (*tick)(void*, int, cudaStream_t)) {
-  k_begin<<<1, 1, 0, s>>>(c->st.p);
+  // the step kernel ends the dt part itself unless bounds of imports or other ranks follow it
+  bool finish = c->owned.empty();
+  for (int p = 0; p < c->P.nfam; ++p) finish = finish && !c->fam[p].have_imp;
   {
     DtArgs a;
     memset(&a, 0, sizeof a);
-    a.nf = c->P.nfam; a.ramp = c->P.cfl_ramp_iter; a.ndir = c->P.ndir;
+    a.nf = c->P.nfam; a.ramp = c->P.cfl_ramp_iter; a.ndir = c->P.ndir; a.time_accurate = c->P.time_accurate;
     a.cfl = c->P.cfl; a.dt_max = c->P.dt_max; a.tau_factor = c->P.tau_factor;
     for (int p = 0; p < c->P.nfam; ++p) {
       FamDev F = make_famdev(c, p, 1, phase);
       a.f[p].Up = F.Up; a.f[p].tau = F.tau; a.f[p].coupled = F.coupled; a.f[p].closure = c->fam[p].closure;
       a.f[p].dt_out = c->P.time_accurate ? nullptr : c->fam[p].dt.p;
     }
-    k_dt_all<<<GRID(c->NI, 256), 256, 0, s>>>(make_geo(c), a, c->st.p);
+    k_dt_all<<<GRID(c->NI, 256), 256, 0, s>>>(make_geo(c), a, finish ? 1 : 0, c->st.p);
   }
   for (int p = 0; p < c->P.nfam; ++p) launch_dt_bounds(c, p, phase, s);
   if (!c->owned.empty() && !c->xerr) {
@@ -538,7 +540,7 @@ static void enqueue_step_dt(ice_gpu_ctx* c, int phase, cudaStream_t s, void (*ti
       cudaStreamSynchronize(s);
     }
   }
-  k_time<<<1, 1, 0, s>>>(c->st.p, c->P.time_accurate);
+  if (!finish) k_time<<<1, 1, 0, s>>>(c->st.p, c->P.time_accurate);
   if (tick) tick(c, KC_DT, s);
 }
 
@@ -566,7 +568,9 @@ static void prof_tick(void* vc, int cls, cudaStream_t s) {
 }
 
 static long long launches_per_step(const ice_gpu_ctx* c) {
-  long long n = 3;
+  bool finish = c->owned.empty();
+  for (int p = 0; p < c->P.nfam; ++p) finish = finish && !c->fam[p].have_imp;
+  long long n = finish ? 1 : 2;
   for (int p = 0; p < c->P.nfam; ++p) n += c->fam[p].have_imp ? 3 : 0;
   for (int p = 0; p < c->P.nfam; ++p) {
     const FamHost& H = c->fam[p];
@@ -806,6 +810,7 @@ int ice_gpu_create(const ice_gpu_params* P, int32_t nblocks, const int32_t* dims
   }
   CKC(c->st.alloc(1));
   Status s0; memset(&s0, 0, sizeof s0);
+  s0.dtbits = kDtStart;
   CKC(cudaMemcpy(c->st.p, &s0, sizeof s0, cudaMemcpyHostToDevice));
   CKC(cudaEventCreate(&c->ev0)); CKC(cudaEventCreate(&c->ev1));
 #undef CKC

@@ -178,6 +178,9 @@ __device__ __forceinline__ void decode(const DBlock& B, long long q, int& i, int
 // moduli are formed once, when the metrics are set (k_rows: the scaled norm and the divisions were two
 // thirds of the kernel's instructions), and the signal speeds' and the rate's quotients are branchless:
 // IG, 128 x 126 x 129 cells: 122 us before, 89 now.
+// The minimum's start value, 1e+5 in single precision (Mod_Explicit.f90:40-44), as bits.
+constexpr unsigned long long kDtStart = 0x40f86a0000000000ull;
+
 struct DtFam {
   const double* Up;
   const double* tau;
@@ -186,7 +189,7 @@ struct DtFam {
 };
 struct DtArgs {
   DtFam f[ICE_GPU_MAX_FAMILIES];
-  int nf, ramp, ndir;
+  int nf, ramp, ndir, time_accurate;
   double cfl, dt_max, tau_factor;
 };
 
@@ -262,7 +265,19 @@ __device__ __forceinline__ double family_dt(const Geo& G, const DtFam& f, const 
   return dt;
 }
 
-__global__ void __launch_bounds__(256, 4) k_dt_all(Geo G, DtArgs a, Status* st) {
+// The end of the dt part of a step (Mod_Explicit.f90:40-44, 67-73): the step's dt, the time, the counters, and
+// the minimum's start value for the next step.
+__device__ __forceinline__ void finish_dt(Status* st, int time_accurate) {
+  const double d = __longlong_as_double((long long)atomicAdd(&st->dtbits, 0ull));   // past L1: other CTAs' minima
+  st->dtglobal = d;
+  if (time_accurate) st->time = st->time + d;
+  st->iter += 1;
+  st->iter_from_call += 1;
+  st->dtbits = kDtStart;
+}
+
+// finish: the last CTA to give its minimum ends the dt part (no bounds of imports or other ranks follow).
+__global__ void __launch_bounds__(256, 4) k_dt_all(Geo G, DtArgs a, int finish, Status* st) {
   long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   double dt = INFINITY;
   const int bq = q < G.NI ? find_block(G.blk, G.nb, q) : 0;
@@ -276,7 +291,7 @@ __global__ void __launch_bounds__(256, 4) k_dt_all(Geo G, DtArgs a, Status* st) 
     for (int d = 0; d < 3; ++d)
 #pragma unroll
       for (int m = 0; m < 4; ++m) vs[d][m] = d < a.ndir ? G.row[(long long)(4 * d + m) * G.NI + q] : 0.0;
-    const int it = st->iter;
+    const int it = st->iter + 1;
     for (int p = 0; p < a.nf; ++p) {
       const DtFam& f = a.f[p];
       double d = f.closure == ICE_CLOSURE_MK ? family_dt<MK>(G, f, a, q, g, vs, it)
@@ -295,7 +310,19 @@ __global__ void __launch_bounds__(256, 4) k_dt_all(Geo G, DtArgs a, Status* st) 
     unsigned long long m = wmin[0];
     for (int w = 1; w < (int)(blockDim.x >> 5); ++w) m = min(m, wmin[w]);
     atomicMin(&st->dtbits, m);
+    if (finish) {
+      __threadfence();
+      if (atomicAdd(&st->done, 1u) == gridDim.x - 1) {
+        __threadfence();
+        st->done = 0u;
+        finish_dt(st, a.time_accurate);
+      }
+    }
   }
+}
+
+__global__ void k_time(Status* st, int time_accurate) {
+  finish_dt(st, time_accurate);
 }
 
 // The rate of compute_dt_ (Mod_dt.f90:256-275): sum over the resolved directions of (|u . versor| +
@@ -1007,20 +1034,6 @@ __global__ void k_update(Geo G, FamDev F, Status* st) {
   if (!check_prim<CL, double>(p)) atomicOr(&st->flags, (unsigned)ICE_GPU_ST_NAN_STATE);
 #pragma unroll
   for (int v = 0; v < nc; ++v) F.Uo[(long long)v * G.NG + g] = p[v];
-}
-
-
-__global__ void k_begin(Status* st) {
-  st->iter += 1;
-  st->iter_from_call += 1;
-  double d = (double)1e+5f;
-  st->dtbits = (unsigned long long)__double_as_longlong(d);
-}
-
-__global__ void k_time(Status* st, int time_accurate) {
-  double d = __longlong_as_double((long long)st->dtbits);
-  st->dtglobal = d;
-  if (time_accurate) st->time = st->time + d;
 }
 
 

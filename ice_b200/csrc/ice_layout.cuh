@@ -65,7 +65,7 @@ constexpr unsigned kNoGhost = 0xffffffffu;
 
 struct Status {
   unsigned int flags;
-  unsigned int pad;
+  unsigned int done;          // CTAs of the step kernel that have given their minimum (k_dt_all)
   unsigned long long nfloored;
   unsigned long long dtbits;  // running min of dt as the bits of a positive double
   double dtglobal;
