@@ -106,49 +106,34 @@ __device__ bool record_flux(const Geo& G, const FamDev& F, const DRec& r, double
   R dl_g1 = cell_length<R>(G, dir, ridx(B, ig, jg, kg));
   R dl_m = cell_length<R>(G, dir, ridx(B, i, j, k));
   R dl_4 = cell_length<R>(G, dir, ridx(B, ip, jp, kp));
-  R dl0, dl1, dl2, dll, dlr;
-  R pl[nc], pr[nc], fl[nc];
-  bool bad;
+  // the stencil in the order of the direction: ghost 2, ghost 1, the cell, its inner neighbour below a face of
+  // odd number, the other way round above one of even number (one code for both: the records of a run's two
+  // ends share warps)
+  const bool odd = f % 2 == 1;
+  const bool ig_inj = F.inj[gidx(B, ig, jg, kg)], ip_inj = F.inj[gidx(B, ip, jp, kp)];
+  const R dl_out = dl_g1;                                               // ghost 2 to ghost 1
+  const R dl_face = ig_inj ? (R)0.5*dl_m : odd ? (R)0.5*(dl_g1 + dl_m) : (R)0.5*(dl_m + dl_g1);
+  const R dl_in = ip_inj ? (R)0.5*dl_m : odd ? (R)0.5*(dl_m + dl_4) : (R)0.5*(dl_4 + dl_m);
+  const R half_g = ig_inj ? (R)0 : (R)0.5*dl_g1, half_m = (R)0.5*dl_m;
+  const R dl0 = odd ? dl_out : dl_in, dl1 = dl_face, dl2 = odd ? dl_in : dl_out;
+  const R dll = odd ? half_g : half_m, dlr = odd ? half_m : half_g;
+  const long long step = odd ? gidx(B, ip, jp, kp) - gidx(B, i, j, k) : gidx(B, ig, jg, kg) - gidx(B, i, j, k);
+  const long long a0 = odd ? gidx(B, ig2, jg2, kg2) : gidx(B, ip, jp, kp);
+  const int c = dir == 0 ? i : dir == 1 ? j : k;
+  const long long fi = fidx(B, dir, i, j, k, odd ? c : c + 1);         // the face below the cell, or above it
+  R nrm[3], area;
+  face_geometry<R>(G, dir, fi, nrm, area);
   const double* P = F.Up;
-  if (f % 2 == 1) {
-    long long fi = fidx(B, dir, i, j, k, (dir == 0 ? i : dir == 1 ? j : k));   // the face below the cell
-    R nrm[3], area;
-    face_geometry<R>(G, dir, fi, nrm, area);
-    dl0 = dl_g1; dl1 = (R)0.5*(dl_g1 + dl_m); dl2 = (R)0.5*(dl_m + dl_4);
-    dll = (R)0.5*dl_g1; dlr = (R)0.5*dl_m;
-    if (F.inj[gidx(B, ig, jg, kg)]) { dl1 = (R)0.5*dl_m; dll = (R)0; }
-    if (F.inj[gidx(B, ip, jp, kp)]) dl2 = (R)0.5*dl_m;
-    long long a[4] = {gidx(B, ig2, jg2, kg2), gidx(B, ig, jg, kg), gidx(B, i, j, k), gidx(B, ip, jp, kp)};
-    R stn[4][nc];
+  R stn[4][nc], pl[nc], pr[nc], fl[nc];
 #pragma unroll
-    for (int s4 = 0; s4 < 4; ++s4)
+  for (int s4 = 0; s4 < 4; ++s4)
 #pragma unroll
-      for (int v = 0; v < nc; ++v) stn[s4][v] = (R)P[(long long)v * G.NG + a[s4]];
-    auto q = [&](int s, int v) { return stn[s][v]; };
-    bad = reconstruct<CL, LIM, R>(F.limiter, q, dl0, dl1, dl2, dll, dlr, pl, pr, bv);
-    riemann<CL, RS, R>(pl, pr, nrm, fl, (R)F.mat.cp);
+    for (int v = 0; v < nc; ++v) stn[s4][v] = (R)P[(long long)v * G.NG + a0 + s4 * step];
+  auto q = [&](int s, int v) { return stn[s][v]; };
+  const bool bad = reconstruct<CL, LIM, R>(F.limiter, q, dl0, dl1, dl2, dll, dlr, pl, pr, bv);
+  riemann<CL, RS, R>(pl, pr, nrm, fl, (R)F.mat.cp);
 #pragma unroll
-    for (int v = 0; v < nc; ++v) flux[v] = (double)(fl[v] * area);
-  } else {
-    long long fi = fidx(B, dir, i, j, k, (dir == 0 ? i : dir == 1 ? j : k) + 1);  // the face above the cell
-    R nrm[3], area;
-    face_geometry<R>(G, dir, fi, nrm, area);
-    dl0 = (R)0.5*(dl_4 + dl_m); dl1 = (R)0.5*(dl_m + dl_g1); dl2 = dl_g1;
-    dll = (R)0.5*dl_m; dlr = (R)0.5*dl_g1;
-    if (F.inj[gidx(B, ig, jg, kg)]) { dl1 = (R)0.5*dl_m; dlr = (R)0; }
-    if (F.inj[gidx(B, ip, jp, kp)]) dl0 = (R)0.5*dl_m;
-    long long a[4] = {gidx(B, ip, jp, kp), gidx(B, i, j, k), gidx(B, ig, jg, kg), gidx(B, ig2, jg2, kg2)};
-    R stn[4][nc];
-#pragma unroll
-    for (int s4 = 0; s4 < 4; ++s4)
-#pragma unroll
-      for (int v = 0; v < nc; ++v) stn[s4][v] = (R)P[(long long)v * G.NG + a[s4]];
-    auto q = [&](int s, int v) { return stn[s][v]; };
-    bad = reconstruct<CL, LIM, R>(F.limiter, q, dl0, dl1, dl2, dll, dlr, pl, pr, bv);
-    riemann<CL, RS, R>(pl, pr, nrm, fl, (R)F.mat.cp);
-#pragma unroll
-    for (int v = 0; v < nc; ++v) flux[v] = (double)(-(fl[v] * area));
-  }
+  for (int v = 0; v < nc; ++v) flux[v] = odd ? (double)(fl[v] * area) : (double)(-(fl[v] * area));
   return bad;
 }
 

@@ -515,6 +515,18 @@ __device__ __forceinline__ void limited(int lim, const R* x, const R* y, R cx, R
   }
 }
 
+// slope_bounds: the limiter's bounds of a cell, its distances to the next cells over its half length.
+template <typename R> __device__ __forceinline__ void limiter_bounds(R dlf, R dlb, R dlc, R& cx, R& cy) {
+  if (dlc > (R)0) {
+    if constexpr (sizeof(R) == 8) {
+      bool ok = ice_div_by(dlc) && dividend(dlf) && dividend(dlb);
+      const R y = ice_div_recip(dlc);
+      cx = ice_div_quot(dlf, dlc, y); cy = ice_div_quot(dlb, dlc, y);
+      if (!ok) { cx = quot_any(dlf, dlc); cy = quot_any(dlb, dlc); }
+    } else { cx = dlf/dlc; cy = dlb/dlc; }
+  } else { cx = (R)2; cy = (R)2; }
+}
+
 // The four cells of a stencil: a source of values q(s, v), s = 0..3 (prev, local, next, next2).
 // state_reconstruction + slope_bounds; returns true when the first-order fallback is itself
 // unphysical (report_stencil).
@@ -523,8 +535,8 @@ __device__ __forceinline__ bool reconstruct(int lim, const Q& q, R dl0, R dl1, R
                                             R* pl, R* pr, R beta) {
   constexpr int nc = NC<CL>::v;
   R cxl, cyl, cxr, cyr, limval = beta;
-  if (dll > (R)0) { cxl = dl1/dll; cyl = dl0/dll; } else { cxl = (R)2; cyl = (R)2; }
-  if (dlr > (R)0) { cxr = dl2/dlr; cyr = dl1/dlr; } else { cxr = (R)2; cyr = (R)2; }
+  limiter_bounds<R>(dl1, dl0, dll, cxl, cyl);
+  limiter_bounds<R>(dl2, dl1, dlr, cxr, cyr);
   const R re = (R)kRhoEmpty;
   R r0 = q(0, 0), r1 = q(1, 0), r2 = q(2, 0), r3 = q(3, 0);
   bool first_l = r0 <= re || r1 <= re || r2 <= re;
@@ -720,6 +732,26 @@ template <int CL, typename R> __device__ __forceinline__ void rusanov(const R* p
   }
 }
 
+// x[v] / d of every v: in FP64 branchless, one reciprocal for all.
+template <int n, typename R> __device__ __forceinline__ void over(R* x, R d) {
+  if constexpr (sizeof(R) == 4) {
+#pragma unroll
+    for (int v = 0; v < n; ++v) x[v] = x[v] / d;
+  } else {
+    const R y = ice_div_recip(d);
+    bool ok = ice_div_by(d);
+#pragma unroll
+    for (int v = 0; v < n; ++v) ok = ok && dividend(x[v]);
+    if (ok) {
+#pragma unroll
+      for (int v = 0; v < n; ++v) x[v] = ice_div_quot(x[v], d, y);
+    } else {
+#pragma unroll
+      for (int v = 0; v < n; ++v) x[v] = quot_any(x[v], d);
+    }
+  }
+}
+
 template <int CL, typename R> __device__ __forceinline__ void hlle(const R* p1, const R* p4, const R* n, R* f, R cp) {
   constexpr int nc = NC<CL>::v;
   R vn1 = p1[1]*n[0] + p1[2]*n[1] + p1[3]*n[2];
@@ -727,11 +759,10 @@ template <int CL, typename R> __device__ __forceinline__ void hlle(const R* p1, 
   R s1, s4;
   wavespeeds<CL, R>(p1, p4, n, s1, s4);
   R r1 = sqrt(p1[0]), r4 = sqrt(p4[0]);
-  R uR = (r1*p1[1] + r4*p4[1]) / (r1 + r4);
-  R vR = (r1*p1[2] + r4*p4[2]) / (r1 + r4);
-  R wR = (r1*p1[3] + r4*p4[3]) / (r1 + r4);
-  R vnR = uR*n[0] + vR*n[1] + wR*n[2];
-  R sR = (r1*s1 + r4*s4) / (r1 + r4);
+  R roe[4] = {r1*p1[1] + r4*p4[1], r1*p1[2] + r4*p4[2], r1*p1[3] + r4*p4[3], r1*s1 + r4*s4};
+  over<4, R>(roe, r1 + r4);
+  R vnR = roe[0]*n[0] + roe[1]*n[1] + roe[2]*n[2];
+  R sR = roe[3];
   R S1 = mn(mn((R)0, vn1 - s1), vnR - sR);
   R S4 = mx(mx((R)0, vn4 + s4), vnR + sR);
   R a0 = -S1, a1 = S1*S4, a2 = S4;
@@ -753,7 +784,8 @@ template <int CL, typename R> __device__ __forceinline__ void hlle(const R* p1, 
     } else {
       flux_make<CL>(p1, n, f1, cp); flux_make<CL>(p4, n, f4, cp);
 #pragma unroll
-      for (int v = 0; v < nc; ++v) f[v] = (S4*f1[v] - S1*f4[v] + S1*S4*(c4[v] - c1[v])) / (S4 - S1);
+      for (int v = 0; v < nc; ++v) f[v] = S4*f1[v] - S1*f4[v] + S1*S4*(c4[v] - c1[v]);
+      over<nc, R>(f, S4 - S1);
     }
   }
 }

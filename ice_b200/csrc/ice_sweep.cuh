@@ -42,14 +42,7 @@ template <int CL, int LIM, typename R>
 __device__ __forceinline__ void slope_of(int lim, const R* sf, const R* sb, R dlf, R dlb, R dlc, bool first, bool fast,
                                          R* s) {
   R cx, cy;
-  if (dlc > (R)0) {
-    if constexpr (sizeof(R) == 8) {
-      bool ok = ice_div_by(dlc) && dividend(dlf) && dividend(dlb);
-      const R y = ice_div_recip(dlc);
-      cx = ice_div_quot(dlf, dlc, y); cy = ice_div_quot(dlb, dlc, y);
-      if (!ok) { cx = quot_any(dlf, dlc); cy = quot_any(dlb, dlc); }
-    } else { cx = dlf/dlc; cy = dlb/dlc; }
-  } else { cx = (R)2; cy = (R)2; }
+  limiter_bounds<R>(dlf, dlb, dlc, cx, cy);
   limited<NC<CL>::v, LIM, R>(lim, sf, sb, cx, cy, first, fast, s);
 }
 
