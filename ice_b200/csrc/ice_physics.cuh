@@ -95,6 +95,29 @@ __device__ __forceinline__ double quot(double a, double b, bool& ok) {
   return ice_div_quot(a, b, ice_div_recip(b));
 }
 
+// The general quotient, out of line: the operands ice_div.h does not take.
+static __device__ __noinline__ double quot_any(double a, double b) { return a / b; }
+
+// x[v] / d of every v: in FP64 branchless, one reciprocal for all.
+template <int n, typename R> __device__ __forceinline__ void over(R* x, R d) {
+  if constexpr (sizeof(R) == 4) {
+#pragma unroll
+    for (int v = 0; v < n; ++v) x[v] = x[v] / d;
+  } else {
+    const R y = ice_div_recip(d);
+    bool ok = ice_div_by(d);
+#pragma unroll
+    for (int v = 0; v < n; ++v) ok = ok && dividend(x[v]);
+    if (ok) {
+#pragma unroll
+      for (int v = 0; v < n; ++v) x[v] = ice_div_quot(x[v], d, y);
+    } else {
+#pragma unroll
+      for (int v = 0; v < n; ++v) x[v] = quot_any(x[v], d);
+    }
+  }
+}
+
 // Limiters the kernels specialise at compile time; any other runs through the run-time switch.
 constexpr int LIM_ANY = -1;
 
@@ -159,6 +182,12 @@ template <int CL> __device__ __forceinline__ void prim2cons_fma(const double* p,
   }
 }
 
+// x / d, as a division in the FP32-flux form (FAST), branchless otherwise: the same value.
+template <bool FAST> __device__ __forceinline__ void temperature(double& x, double d) {
+  if constexpr (FAST) x = x / d;
+  else over<1, double>(&x, d);
+}
+
 // cons -> prim with the reference's floors (Lib_Model_*: cons_2_prim_*). FAST (the FP32-flux form):
 // the velocities multiply by one reciprocal of the density instead of three divisions, and the fused
 // multiply-adds of the speed are written out, as in prim2cons_fma.
@@ -169,13 +198,15 @@ template <int CL, bool FAST = false> __device__ __forceinline__ void cons2prim(c
     const double inv = 1.0 / (p[0] + eps);
     p[1] = c[1] * inv; p[2] = c[2] * inv; p[3] = c[3] * inv;
   } else {
-    p[1] = c[1] / (p[0] + eps); p[2] = c[2] / (p[0] + eps); p[3] = c[3] / (p[0] + eps);
+    p[1] = c[1]; p[2] = c[2]; p[3] = c[3];
+    over<3, double>(p + 1, p[0] + eps);
   }
   double n2;
   if constexpr (FAST) n2 = __fma_rn(p[3], p[3], __fma_rn(p[2], p[2], __dmul_rn(p[1], p[1])));
   else n2 = p[1]*p[1] + p[2]*p[2] + p[3]*p[3];
   if constexpr (CL == MK) {
-    p[4] = (c[4] - 0.5*p[0]*n2) / (cp*p[0] + eps);
+    p[4] = c[4] - 0.5*p[0]*n2;
+    temperature<FAST>(p[4], cp*p[0] + eps);
     p[5] = c[5];
     if (p[0] < eps) {
 #pragma unroll
@@ -186,7 +217,8 @@ template <int CL, bool FAST = false> __device__ __forceinline__ void cons2prim(c
   } else if constexpr (CL == IG) {
     p[4] = 1.0/3.0 * (c[4] - p[0]*n2);
     if (p[0] <= kRhoEmpty && p[4] > p[0]*kThetaCap) p[4] = p[0]*kThetaCap;
-    p[5] = (c[5] - 0.5*c[4]) / (cp*p[0] + eps);
+    p[5] = c[5] - 0.5*c[4];
+    temperature<FAST>(p[5], cp*p[0] + eps);
     p[6] = c[6];
     if (p[0] < eps) {
 #pragma unroll
@@ -202,7 +234,8 @@ template <int CL, bool FAST = false> __device__ __forceinline__ void cons2prim(c
     p[7] = c[7] - p[0]*p[2]*p[2];
     p[8] = c[8] - p[0]*p[2]*p[3];
     p[9] = c[9] - p[0]*p[3]*p[3];
-    p[10] = (c[10] - 0.5*(c[4] + c[7] + c[9])) / (cp*p[0] + eps);
+    p[10] = c[10] - 0.5*(c[4] + c[7] + c[9]);
+    temperature<FAST>(p[10], cp*p[0] + eps);
     p[11] = c[11];
     if (p[0] <= kRhoEmpty && p[4] + p[7] + p[9] > 3.0*p[0]*kThetaCap) {
       double f = 3.0*p[0]*kThetaCap / (p[4] + p[7] + p[9]);
@@ -423,8 +456,7 @@ template <int LIM, typename R> __device__ __forceinline__ R limiter(int lim, R x
   return phi * x;
 }
 
-// The general forms, out of line: the operands ice_div.h does not take.
-static __device__ __noinline__ double quot_any(double a, double b) { return a / b; }
+// The limiter's general form, out of line.
 static __device__ __noinline__ double limiter_any(int lim, double x, double y, double cx, double cy) {
   return limiter<LIM_ANY, double>(lim, x, y, cx, cy);
 }
@@ -729,26 +761,6 @@ template <int CL, typename R> __device__ __forceinline__ void rusanov(const R* p
     flux_make<CL>(p1, n, f1, cp); flux_make<CL>(p4, n, f4, cp);
 #pragma unroll
     for (int v = 0; v < nc; ++v) f[v] = (R)0.5 * (f1[v] + f4[v] - A*(c4[v] - c1[v]));
-  }
-}
-
-// x[v] / d of every v: in FP64 branchless, one reciprocal for all.
-template <int n, typename R> __device__ __forceinline__ void over(R* x, R d) {
-  if constexpr (sizeof(R) == 4) {
-#pragma unroll
-    for (int v = 0; v < n; ++v) x[v] = x[v] / d;
-  } else {
-    const R y = ice_div_recip(d);
-    bool ok = ice_div_by(d);
-#pragma unroll
-    for (int v = 0; v < n; ++v) ok = ok && dividend(x[v]);
-    if (ok) {
-#pragma unroll
-      for (int v = 0; v < n; ++v) x[v] = ice_div_quot(x[v], d, y);
-    } else {
-#pragma unroll
-      for (int v = 0; v < n; ++v) x[v] = quot_any(x[v], d);
-    }
   }
 }
 
