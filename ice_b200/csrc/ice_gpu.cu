@@ -178,6 +178,8 @@ struct ice_gpu_ctx {
   unsigned long long xbits = 0;  // the reduced dt on its way back to the device
   long long nlaunch = 0;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+  cudaEvent_t t0 = nullptr, t1 = nullptr;   // around a call's steps
+  Status* hst = nullptr;    // the status as the last call's steps left it (page-locked)
   DevBuf<double> xfer;    // one block of one family in the caller's layout (upload/download)
   long long ng_max = 0;
   std::string err;
@@ -813,6 +815,8 @@ int ice_gpu_create(const ice_gpu_params* P, int32_t nblocks, const int32_t* dims
   s0.dtbits = kDtStart;
   CKC(cudaMemcpy(c->st.p, &s0, sizeof s0, cudaMemcpyHostToDevice));
   CKC(cudaEventCreate(&c->ev0)); CKC(cudaEventCreate(&c->ev1));
+  CKC(cudaEventCreate(&c->t0)); CKC(cudaEventCreate(&c->t1));
+  CKC(cudaMallocHost((void**)&c->hst, sizeof(Status)));
 #undef CKC
   if (build_tiles(c)) { g_create_err = c->err; return ICE_GPU_ECUDA; }
   *out = u.release();
@@ -825,6 +829,9 @@ int ice_gpu_destroy(ice_gpu_ctx* c) {
   free_graphs(c);
   if (c->ev0) cudaEventDestroy(c->ev0);
   if (c->ev1) cudaEventDestroy(c->ev1);
+  if (c->t0) cudaEventDestroy(c->t0);
+  if (c->t1) cudaEventDestroy(c->t1);
+  if (c->hst) cudaFreeHost(c->hst);
   if (c->s_up) { cudaStreamSynchronize(c->s_up); cudaStreamDestroy(c->s_up); }
   if (c->s_down) { cudaStreamSynchronize(c->s_down); cudaStreamDestroy(c->s_down); }
   if (c->ev_up) cudaEventDestroy(c->ev_up);
@@ -1393,7 +1400,7 @@ static int check_ready(ice_gpu_ctx* c) {
   return 0;
 }
 
-static int finish_step(ice_gpu_ctx* c, ice_gpu_step_out* out, float dms);
+static int finish_step(ice_gpu_ctx* c, ice_gpu_step_out* out);
 
 int ice_gpu_step(ice_gpu_ctx* c, int32_t nsteps, ice_gpu_step_out* out) {
   if (!c) return ICE_GPU_EINVAL;
@@ -1411,9 +1418,7 @@ int ice_gpu_step(ice_gpu_ctx* c, int32_t nsteps, ice_gpu_step_out* out) {
   // call ends at the step that meets it
   const bool res_stop = !c->P.time_accurate && c->P.res_threshold > 0.0;
   c->res_end = false;
-  cudaEvent_t t0 = nullptr, t1 = nullptr;
-  CK(cudaEventCreate(&t0)); CK(cudaEventCreate(&t1));
-  CK(cudaEventRecord(t0, s));
+  CK(cudaEventRecord(c->t0, s));
   for (int n = 0; n < nsteps && !c->res_end; ++n) {
     int ph = c->phase;
     if (c->profiling) {
@@ -1426,7 +1431,6 @@ int ice_gpu_step(ice_gpu_ctx* c, int32_t nsteps, ice_gpu_step_out* out) {
       enqueue_step(c, ph, s, nullptr);
       if (c->xerr) {
         cudaStreamSynchronize(s);
-        cudaEventDestroy(t0); cudaEventDestroy(t1);
         return c->xerr;
       }
     } else {
@@ -1443,27 +1447,23 @@ int ice_gpu_step(ice_gpu_ctx* c, int32_t nsteps, ice_gpu_step_out* out) {
     c->prev_phase = ph;
     c->phase = next_phase(c, ph);
     if (res_stop) {
-      if (int rc = ice_gpu_residual_norm(c, c->last_norm, nullptr)) {
-        cudaEventDestroy(t0); cudaEventDestroy(t1);
-        return rc;
-      }
+      if (int rc = ice_gpu_residual_norm(c, c->last_norm, nullptr)) return rc;
       if (c->res_reference == 0.0) c->res_reference = c->last_norm[0];
       c->res_end = c->res_reference > 0.0 && c->last_norm[0] <= c->P.res_threshold * c->res_reference;
     }
   }
-  CK(cudaEventRecord(t1, s));
+  CK(cudaEventRecord(c->t1, s));
+  CK(cudaMemcpyAsync(c->hst, c->st.p, sizeof(Status), cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
-  float dms = 0.f;
-  CK(cudaEventElapsedTime(&dms, t0, t1));
-  cudaEventDestroy(t0); cudaEventDestroy(t1);
-  return finish_step(c, out, dms);
+  return finish_step(c, out);
 }
 
-// The step's report from the device status (after the stream has drained).
-static int finish_step(ice_gpu_ctx* c, ice_gpu_step_out* out, float dms) {
+// The step's report from the status the call copied after its steps (the stream has drained).
+static int finish_step(ice_gpu_ctx* c, ice_gpu_step_out* out) {
   CK(cudaGetLastError());
-  Status h;
-  CK(cudaMemcpy(&h, c->st.p, sizeof h, cudaMemcpyDeviceToHost));
+  const Status& h = *c->hst;
+  float dms = 0.f;
+  CK(cudaEventElapsedTime(&dms, c->t0, c->t1));
   int rc = 0;
   if (out) {
     out->dtglobal = h.dtglobal; out->time = h.time; out->iter = h.iter; out->status = (int)h.flags;
@@ -1532,9 +1532,7 @@ int ice_gpu_step_host(ice_gpu_ctx* c, int32_t nsteps, const double* const* prim_
   std::vector<int> order(nf);
   for (int p = 0; p < nf; ++p) order[p] = p;
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return c->fam[a].nc > c->fam[b].nc; });
-  cudaEvent_t t0 = nullptr, t1 = nullptr;
-  CK(cudaEventCreate(&t0)); CK(cudaEventCreate(&t1));
-  CK(cudaEventRecord(t0, c->s_up));
+  CK(cudaEventRecord(c->t0, c->s_up));
   const int ph0 = c->phase;
   for (int p : order)
     for (int b = 0; b < c->nb; ++b) {
@@ -1594,13 +1592,11 @@ int ice_gpu_step_host(ice_gpu_ctx* c, int32_t nsteps, const double* const* prim_
     c->prev_phase = ph;
     c->phase = phn;
   }
-  CK(cudaEventRecord(t1, c->s_down));
+  CK(cudaMemcpyAsync(c->hst, c->st.p, sizeof(Status), cudaMemcpyDeviceToHost, s));
+  CK(cudaEventRecord(c->t1, c->s_down));
   CK(cudaStreamSynchronize(c->s_down));
   CK(cudaStreamSynchronize(s));
-  float dms = 0.f;
-  CK(cudaEventElapsedTime(&dms, t0, t1));
-  cudaEventDestroy(t0); cudaEventDestroy(t1);
-  return finish_step(c, out, dms);
+  return finish_step(c, out);
 }
 
 int ice_gpu_residual_norm(ice_gpu_ctx* c, double* total, double* fam) {
