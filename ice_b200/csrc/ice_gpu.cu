@@ -633,8 +633,8 @@ static int build_sweeps(ice_gpu_ctx* c) {
   for (int p = 0; p < c->P.nfam; ++p) {
     FamHost& H = c->fam[p];
     const TuneRow tr = tune_of(H.closure);
-    const int occ = H.closure == ICE_CLOSURE_AG ? (f64 ? SweepOcc<AG, double>::v : SweepOcc<AG, float>::v)
-                                                : (f64 ? SweepOcc<MK, double>::v : SweepOcc<MK, float>::v);
+    const int occ = H.closure == ICE_CLOSURE_AG ? (f64 ? SweepOcc<AG, double>::flux : SweepOcc<AG, float>::flux)
+                                                : (f64 ? SweepOcc<MK, double>::flux : SweepOcc<MK, float>::flux);
     const double slots = (double)nsm * occ * SW_NT;
     const int cy = choose_march(c, 1, slots, tr), cz = choose_march(c, 2, slots, tr);
     std::vector<SweepJob> f;

@@ -31,10 +31,13 @@ namespace ice {
 constexpr int SW_NT = 128;                      // threads per CTA
 constexpr int SW_XC = SW_NT / 32 * 31;          // cells whose upper x face one CTA computes
 
-// The CTAs per SM the kernels are held to: in FP64 128 registers for MK and IG, 255 for AG, whose twelve
-// variables would otherwise spill; in the FP32-flux form 96 and 128.
+// The CTAs per SM the flux and the cell kernel are held to. Flux: 6 against 5 in the FP32-flux form 192 / 214 us
+// (IG, 128 x 126 x 129; AG at 6 spills, 209 / 164 us on 96^3), 3 against 2 for FP64 AG 152 / 160 us
+// (64 x 61 x 67), 4 against 3 and 5 for FP64 IG 225 / 248 / 246 us (96 x 95 x 97). Cells: 5 against 6 139 / 145 us
+// (FP32 IG), AG 2 against 3 56 / 69 us (FP64): its loads are what it holds registers for.
 template <int CL, typename R> struct SweepOcc {
-  static constexpr int v = sizeof(R) == 8 ? (CL == AG ? 2 : 4) : (CL == AG ? 4 : 5);
+  static constexpr int flux = sizeof(R) == 8 ? (CL == AG ? 3 : 4) : (CL == AG ? 4 : 6);
+  static constexpr int cells = sizeof(R) == 8 ? (CL == AG ? 2 : 4) : (CL == AG ? 4 : 5);
 };
 
 // Limited slope of one cell from its two difference quotients.
@@ -313,7 +316,7 @@ __device__ __forceinline__ void cell_update(const Geo& G, const FamDev& F, long 
 
 // The first nrb CTAs take the boundary records (long chains: they start first), the others a job each.
 template <int CL, int RS, int LIM, typename R>
-__global__ void __launch_bounds__(SW_NT, SweepOcc<CL, R>::v)
+__global__ void __launch_bounds__(SW_NT, SweepOcc<CL, R>::flux)
 k_flux(Geo G, FamDev F, const SweepJob* __restrict__ jobs, const DRec* recs, const int* frec, int nfrec, int nrb, Status* st) {
   bool bad = false;
   if ((int)blockIdx.x < nrb) {
@@ -336,7 +339,7 @@ k_flux(Geo G, FamDev F, const SweepJob* __restrict__ jobs, const DRec* recs, con
 
 // The update of every cell. write_r: store R instead of updating (IRS runs).
 template <int CL, typename R>
-__global__ void __launch_bounds__(SW_NT, SweepOcc<CL, R>::v) k_cells(Geo G, FamDev F, int write_r, Status* st) {
+__global__ void __launch_bounds__(SW_NT, SweepOcc<CL, R>::cells) k_cells(Geo G, FamDev F, int write_r, Status* st) {
   constexpr int nc = NC<CL>::v;
   const long long q = (long long)blockIdx.x * SW_NT + threadIdx.x;
   if (q >= G.NI) return;
