@@ -150,6 +150,10 @@ enum { SW_X = 0, SW_Y = 1, SW_Z = 2 };
 struct SweepJob { int b, kind, base, c0, n; };
 struct NormChunk { int b; long long q0, q1; };
 
+// The parts of a family's stage: what comes before its faces (source, ghosts, sensor), and the faces and the
+// update.
+enum { PART_ALL = 0, PART_PREP, PART_FACES };
+
 // Everything one family's stage needs, for the launcher of its closure's translation unit.
 struct LaunchArgs {
   Geo G;
@@ -164,6 +168,7 @@ struct LaunchArgs {
   const unsigned char* mlp_img;                      // the family's surrogate network (null: the plain closure)
   const MlpNorm* mlp_norm;
   int ndir, sd, irs, precision;
+  int part;                                          // PART_*
   int plane;                                         // the FP32-flux form's 1-D stage kernel runs (ice_kernels.cuh)
   double irs_beta;
   double* resid; double* resid2; double* resid3;
