@@ -791,10 +791,11 @@ __device__ __forceinline__ void edge_sum(const DBlock& B, int i, int j, int k, d
 // at the start of the stage and the frozen gas; written to S (and tau, on the last stage), which
 // the stage kernel adds to the residual. Its own kernel, so that the iterative closures do not
 // share the stencil kernel's registers.
-// 64 registers (4 CTAs per SM) in FP32; in FP64 128 (2): at 64 its deterministic elementary functions spilled
-// 750 bytes a thread, eight times the DRAM writes the source needs.
+// Bound by its chains (four to six powers, the Langmuir-Knudsen iteration), so it wants warps: 64 registers
+// (4 CTAs per SM) against 80 and 128 (3, 2) take 82 / 91 / 95 us in FP64 (evaporating AG, 64 x 61 x 67) although
+// some spill (74 / 74 / 86 us for IG without evaporation, 96 x 95 x 97).
 template <int CL, typename R>
-__global__ void __launch_bounds__(256, sizeof(R) == 8 ? 2 : 4) k_source(Geo G, FamDev F) {
+__global__ void __launch_bounds__(256, 4) k_source(Geo G, FamDev F) {
   constexpr int nc = NC<CL>::v;
   long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= G.NI) return;
