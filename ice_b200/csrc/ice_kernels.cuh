@@ -148,11 +148,13 @@ __device__ __forceinline__ int find_block(const DBlock* blk, int nb, long long q
   return lo;
 }
 
+// The indices of interior cell q of block B, by 32-bit arithmetic (a block has fewer than 2^31 cells; in 64 bits
+// the divisions were half of the sensor kernel's instructions).
 __device__ __forceinline__ void decode(const DBlock& B, long long q, int& i, int& j, int& k) {
-  long long l = q - B.ioff;
-  i = (int)(l % B.ni); l /= B.ni;
-  j = (int)(l % B.nj);
-  k = (int)(l / B.nj);
+  const unsigned l = (unsigned)(q - B.ioff), ni = (unsigned)B.ni, nj = (unsigned)B.nj, jk = l / ni;
+  i = (int)(l % ni);
+  j = (int)(jk % nj);
+  k = (int)(jk / nj);
 }
 
 // compute_dt for every family in one pass (Mod_dt.f90:11-112, 256-275; Mod_Explicit.f90:46-61): each
