@@ -57,12 +57,12 @@ void launch_family_t(const LaunchArgs& a) {
     }
     if (a.xchg) a.xchg(a, ICE_GPU_HALO_CELLS);   // the remote source cells of the ghost layers
     if (a.ngrec + a.ncopy > 0) {
-      const unsigned g = grid((long long)a.ngrec + a.ncopy, 128);
+      const unsigned nrb = grid(a.ngrec, 128), g = nrb + GhostPart<CL>::n * grid(a.ncopy, 128);
       if (a.ghost_split) {
-        k_ghost<CL><<<g, 128, 0, s>>>(a.G, a.F, a.grecs, a.ngrec, 1, nullptr, 0, 0);
-        k_ghost<CL><<<g, 128, 0, s>>>(a.G, a.F, a.grecs, a.ngrec, 2, nullptr, 0, 0);
+        k_ghost<CL><<<g, 128, 0, s>>>(a.G, a.F, a.grecs, a.ngrec, nrb, 1, nullptr, 0, 0);
+        k_ghost<CL><<<g, 128, 0, s>>>(a.G, a.F, a.grecs, a.ngrec, nrb, 2, nullptr, 0, 0);
       } else {
-        k_ghost<CL><<<g, 128, 0, s>>>(a.G, a.F, a.grecs, a.ngrec, 3, a.gcopy, a.ncopy, a.next);
+        k_ghost<CL><<<g, 128, 0, s>>>(a.G, a.F, a.grecs, a.ngrec, nrb, 3, a.gcopy, a.ncopy, a.next);
       }
       tick(KC_GHOST);
     }

@@ -114,6 +114,7 @@ struct FamHost {
 struct ice_gpu_ctx {
   ice_gpu_params P;
   int nb = 0;
+  int nsm = 148;            // the GPU's SMs
   std::vector<int> dims;
   std::vector<DBlock> hblk;
   long long NG = 0, NI = 0, NR = 0, NF[3] = {0, 0, 0};
@@ -527,7 +528,7 @@ static void enqueue_step_dt(ice_gpu_ctx* c, int phase, cudaStream_t s, void (*ti
       a.f[p].Up = F.Up; a.f[p].tau = F.tau; a.f[p].coupled = F.coupled; a.f[p].closure = c->fam[p].closure;
       a.f[p].dt_out = c->P.time_accurate ? nullptr : c->fam[p].dt.p;
     }
-    k_dt_all<<<GRID(c->NI, 256), 256, 0, s>>>(make_geo(c), a, finish ? 1 : 0, c->st.p);
+    k_dt_all<<<std::min(GRID(c->NI, 256), 4u * (unsigned)c->nsm), 256, 0, s>>>(make_geo(c), a, finish ? 1 : 0, c->st.p);
   }
   for (int p = 0; p < c->P.nfam; ++p) launch_dt_bounds(c, p, phase, s);
   if (!c->owned.empty() && !c->xerr) {
@@ -674,16 +675,16 @@ static int choose_march(const ice_gpu_ctx* c, int d, double slots, const TuneRow
 // The flux kernel's CTAs (ice_sweep.cuh) over the owned blocks, by slabs of wcap planes: the x, y and z faces of
 // a slab one after the other, so that the second and third read the state from L2.
 static int build_sweeps(ice_gpu_ctx* c) {
-  int nsm = 148, dev = 0;
+  int dev = 0;
   CK(cudaGetDevice(&dev));
-  CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  CK(cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, dev));
   const bool f64 = c->P.precision != ICE_PREC_FP32FLUX;
   for (int p = 0; p < c->P.nfam; ++p) {
     FamHost& H = c->fam[p];
     const TuneRow tr = tune_of(H.closure);
     const int occ = H.closure == ICE_CLOSURE_AG ? (f64 ? SweepOcc<AG, double>::flux : SweepOcc<AG, float>::flux)
                                                 : (f64 ? SweepOcc<MK, double>::flux : SweepOcc<MK, float>::flux);
-    const double slots = (double)nsm * occ * SW_NT;
+    const double slots = (double)c->nsm * occ * SW_NT;
     const int cy = choose_march(c, 1, slots, tr), cz = choose_march(c, 2, slots, tr);
     std::vector<SweepJob> f;
     std::vector<int> slab;           // per job, its slab of the block

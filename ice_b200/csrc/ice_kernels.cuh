@@ -164,7 +164,9 @@ __device__ __forceinline__ void decode(const DBlock& B, long long q, int& i, int
 // minimum, so the order of the families does not matter). Bound by its reads. The rows' unit vectors and
 // moduli are formed once, when the metrics are set (k_rows: the scaled norm and the divisions were two
 // thirds of the kernel's instructions), and the signal speeds' and the rate's quotients are branchless:
-// IG, 128 x 126 x 129 cells: 122 us before, 89 now.
+// A resident grid strides over the cells: one reduction and one atomic a CTA, not one per 256 cells, behind
+// which the slot stood idle. IG, 128 x 126 x 129 cells: 122 us with the rows formed in the step, 89 with a CTA
+// per 256 cells, 77 now.
 // The minimum's start value, 1e+5 in single precision (Mod_Explicit.f90:40-44), as bits.
 constexpr unsigned long long kDtStart = 0x40f86a0000000000ull;
 
@@ -229,6 +231,8 @@ __device__ __forceinline__ double family_dt(const Geo& G, const DtFam& f, const 
   double p[nc];
 #pragma unroll
   for (int v = 0; v < used; ++v) p[v] = f.Up[(long long)v * G.NG + g];
+  const bool bound = f.coupled && a.tau_factor > 0.0;
+  const double tau = bound ? f.tau[q] : 0.0;     // with the state's loads, not after the rate
   double ws[3], rate = 0.0;
   row_speeds<CL>(p, vs, ws);
 #pragma unroll
@@ -244,10 +248,7 @@ __device__ __forceinline__ double family_dt(const Geo& G, const DtFam& f, const 
   dt = dt * a.cfl;
   if (it <= a.ramp) dt = dt * (double)it / (double)a.ramp;
   dt = mn(dt, a.dt_max);
-  if (f.coupled && a.tau_factor > 0.0) {
-    double tau = f.tau[q];
-    if (p[0] > kRhoEmpty && !not_finite(tau) && tau > 0.0) dt = mn(dt, a.tau_factor*tau);
-  }
+  if (bound && p[0] > kRhoEmpty && !not_finite(tau) && tau > 0.0) dt = mn(dt, a.tau_factor*tau);
   if (f.dt_out) f.dt_out[q] = dt;
   return dt;
 }
@@ -265,20 +266,20 @@ __device__ __forceinline__ void finish_dt(Status* st, int time_accurate) {
 
 // finish: the last CTA to give its minimum ends the dt part (no bounds of imports or other ranks follow).
 __global__ void __launch_bounds__(256, 4) k_dt_all(Geo G, DtArgs a, int finish, Status* st) {
-  long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   double dt = INFINITY;
-  const int bq = q < G.NI ? find_block(G.blk, G.nb, q) : 0;
-  if (q < G.NI && stepped(G, bq)) {
+  const int it = st->iter + 1;
+  for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < G.NI; q += (long long)gridDim.x * blockDim.x) {
+    const int bq = find_block(G.blk, G.nb, q);
+    if (!stepped(G, bq)) continue;
     const DBlock& B = G.blk[bq];
-    const unsigned l = (unsigned)(q - B.ioff), ni = (unsigned)B.ni, nj = (unsigned)B.nj;
-    const unsigned i = l % ni, jk = l / ni, j = jk % nj, k = jk / nj;
-    const long long g = gidx(B, (int)i, (int)j, (int)k);
+    int i, j, k;
+    decode(B, q, i, j, k);
+    const long long g = gidx(B, i, j, k);
     double vs[3][4];
 #pragma unroll
     for (int d = 0; d < 3; ++d)
 #pragma unroll
       for (int m = 0; m < 4; ++m) vs[d][m] = d < a.ndir ? G.row[(long long)(4 * d + m) * G.NI + q] : 0.0;
-    const int it = st->iter + 1;
     for (int p = 0; p < a.nf; ++p) {
       const DtFam& f = a.f[p];
       double d = f.closure == ICE_CLOSURE_MK ? family_dt<MK>(G, f, a, q, g, vs, it)
@@ -638,34 +639,44 @@ __device__ __forceinline__ void ghost2_rec(const Geo& G, const FamDev& F, const 
 // operations of ghost1_rec followed by ghost2_rec (layer 2 of a 400 record, 3 g1 - 3 m + p, with g1 the layer-1
 // value just copied from m). Bound by the records' and cells' bytes: on a 509 x 512 plane, whose 260,608 cells
 // have two k faces each, reading the whole record cost 34 us a launch.
+// An AG thread takes a third of a record's variables, so that more of them wait on memory at once: 45 / 35 us on
+// 8 blocks of 1.7 M cells; MK and IG in two parts gained nothing there and lost 20 % on the plane.
+template <int CL> struct GhostPart {
+  static constexpr int n = CL == AG ? 3 : 1, nv = (NC<CL>::v + n - 1) / n;
+};
+
 template <int CL>
-__device__ __forceinline__ void ghost_copy(double* P, long long NG, const GhostCopy& c, bool ext) {
-  constexpr int nc = NC<CL>::v;
-  double a[nc], b[nc];
+__device__ __forceinline__ void ghost_copy(double* P, long long NG, const GhostCopy& c, bool ext, int v0) {
+  constexpr int nv = GhostPart<CL>::nv, nc = NC<CL>::v;
+  double a[nv], b[nv];
   const bool two = c.g2 != kNoGhost;
+  P += (long long)v0 * NG;
 #pragma unroll
-  for (int v = 0; v < nc; ++v) a[v] = P[v * NG + c.m];
+  for (int v = 0; v < nv; ++v) if (v0 + v < nc) a[v] = P[v * NG + c.m];
   if (two) {
 #pragma unroll
-    for (int v = 0; v < nc; ++v) b[v] = P[v * NG + c.p];
+    for (int v = 0; v < nv; ++v) if (v0 + v < nc) b[v] = P[v * NG + c.p];
   }
 #pragma unroll
-  for (int v = 0; v < nc; ++v) P[v * NG + c.g1] = a[v];
+  for (int v = 0; v < nv; ++v) if (v0 + v < nc) P[v * NG + c.g1] = a[v];
   if (two) {
 #pragma unroll
-    for (int v = 0; v < nc; ++v) P[v * NG + c.g2] = ext ? 3.0*a[v] - 3.0*a[v] + b[v] : b[v];
+    for (int v = 0; v < nv; ++v) if (v0 + v < nc) P[v * NG + c.g2] = ext ? 3.0*a[v] - 3.0*a[v] + b[v] : b[v];
   }
 }
 
-// Threads 0 .. nrec - 1 take the records, the others the copies.
+// The first nrb CTAs take the records, the others the copies, part by part.
 template <int CL>
-__global__ void k_ghost(Geo G, FamDev F, const DRec* recs, int nrec, int layers, const GhostCopy* copies, int ncopy, int next) {
-  int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= nrec) {
-    n -= nrec;
-    if (n < ncopy) ghost_copy<CL>(F.Ug, G.NG, copies[n], n < next);
+__global__ void k_ghost(Geo G, FamDev F, const DRec* recs, int nrec, int nrb, int layers, const GhostCopy* copies, int ncopy,
+                        int next) {
+  if ((int)blockIdx.x >= nrb) {
+    const int ncb = (gridDim.x - nrb) / GhostPart<CL>::n, cb = blockIdx.x - nrb;
+    const int n = (cb % ncb) * blockDim.x + threadIdx.x;
+    if (n < ncopy) ghost_copy<CL>(F.Ug, G.NG, copies[n], n < next, cb / ncb * GhostPart<CL>::nv);
     return;
   }
+  const int n = blockIdx.x * blockDim.x + threadIdx.x;
+  if (n >= nrec) return;
   const DRec r = recs[n];
   if (!stepped(G, r.b)) return;
   if (layers & 1) ghost1_rec<CL>(G, F, r);
