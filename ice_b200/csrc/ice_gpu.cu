@@ -685,6 +685,9 @@ static int build_sweeps(ice_gpu_ctx* c) {
     const int occ = H.closure == ICE_CLOSURE_AG ? (f64 ? SweepOcc<AG, double>::flux : SweepOcc<AG, float>::flux)
                                                 : (f64 ? SweepOcc<MK, double>::flux : SweepOcc<MK, float>::flux);
     const double slots = (double)c->nsm * occ * SW_NT;
+    // groups of SW_XC cells an x CTA takes: the start of a CTA (its job, its block, their loads) is a chain of its
+    // own, 183 / 172 us for one / four groups (FP32 IG, 128 x 126 x 129); one in a run too small for two waves
+    const int cx = (int)std::min(4.0, std::max(1.0, (double)c->NI / (2.0 * slots)));
     const int cy = choose_march(c, 1, slots, tr), cz = choose_march(c, 2, slots, tr);
     std::vector<SweepJob> f;
     std::vector<int> slab;           // per job, its slab of the block
@@ -697,7 +700,7 @@ static int build_sweeps(ice_gpu_ctx* c) {
         slab.push_back(k / tr.wcap);
       };
       if (ni >= 2)
-        for (long long q = 0; q < ncell; q += SW_XC) put(SW_X, q, 0, 0, (int)(q / ((long long)ni * nj)));
+        for (long long q = 0; q < ncell; q += (long long)cx * SW_XC) put(SW_X, q, 0, cx, (int)(q / ((long long)ni * nj)));
       auto chunks = [&](int kind, int n, int len, long long cols) {
         const int nch = (n + len - 1) / len, base = n / nch, extra = n % nch;
         for (long long q = 0; q < cols; q += SW_NT)

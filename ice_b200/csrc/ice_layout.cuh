@@ -143,8 +143,8 @@ struct EmptyScan {
 struct Tile { int b, i0, j0, k0, nkz; };
 struct MlpNorm;
 
-// One CTA's share of the flux kernel (ice_sweep.cuh): the x faces above the cells base.. of block b (flat over
-// the block), or the y or z faces above the cells c0 .. c0 + n - 1 of the columns base.. (flat over the plane
+// One CTA's share of the flux kernel (ice_sweep.cuh): the x faces above n groups of SW_XC cells from base of block
+// b (flat over the block), or the y or z faces above the cells c0 .. c0 + n - 1 of the columns base.. (flat over the plane
 // across them).
 enum { SW_X = 0, SW_Y = 1, SW_Z = 2 };
 struct SweepJob { int b, kind, base, c0, n; };

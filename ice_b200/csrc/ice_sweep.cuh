@@ -327,7 +327,7 @@ k_flux(Geo G, FamDev F, const SweepJob* __restrict__ jobs, const DRec* recs, con
   const SweepJob t = jobs[blockIdx.x - nrb];
   const DBlock B = G.blk[t.b];
   if (t.kind == SW_X) {
-    bad = x_faces<CL, RS, LIM, R>(G, F, B, t.base);
+    for (int m = 0; m < t.n; ++m) bad |= x_faces<CL, RS, LIM, R>(G, F, B, t.base + m * SW_XC);
   } else {
     const int col = t.base + threadIdx.x;
     const bool y = t.kind == SW_Y;
