@@ -41,20 +41,17 @@ void launch_family_t(const LaunchArgs& a) {
   cudaStream_t s = a.s;
   auto tick = [&](int cls) { if (a.tick) a.tick(a.tick_ctx, cls, s); };
   auto grid = [](long long n, int t) { return (unsigned)((n + t - 1) / t); };
-  const bool f32 = a.precision == ICE_PREC_FP32FLUX && !a.irs;
-  if (a.part != PART_FACES) {
-    // compute_source comes first in the stage (Mod_Explicit.f90:111-117). In the FP32-flux form the cells'
-    // kernel evaluates the source of a family without evaporation itself; an evaporating family's source
-    // (iterative, with lane-divergent trip counts) runs in its own kernel at full occupancy, or in the
-    // surrogate's source kernel, and the stage reads it (FamDev::src_ready). So does every FP64 source, whose
-    // deterministic elementary functions would take the cells' kernel's registers, and the plane kernel's.
-    if (a.F.coupled && a.mlp_img) {
-      launch_source_mlp(CL, a, a.mlp_img, *a.mlp_norm);
-      tick(KC_SOURCE);
-    } else if (a.F.coupled && (a.F.src_ready || !f32 || a.plane)) {
-      launch_source_of<CL>(a);
-      tick(KC_SOURCE);
-    }
+  // compute_source comes first in the stage (Mod_Explicit.f90:111-117). In the FP32-flux form the cells'
+  // kernel evaluates the source of a family without evaporation itself; an evaporating family's source
+  // (iterative, with lane-divergent trip counts) runs in its own kernel at full occupancy, or in the
+  // surrogate's source kernel, and the stage reads it (FamDev::src_ready). So does every FP64 source, whose
+  // deterministic elementary functions would take the cells' kernel's registers, and the plane kernel's.
+  if ((a.part & PART_SOURCE) && a.own_source) {
+    if (a.mlp_img) launch_source_mlp(CL, a, a.mlp_img, *a.mlp_norm);
+    else launch_source_of<CL>(a);
+    tick(KC_SOURCE);
+  }
+  if (a.part & PART_GHOSTS) {
     if (a.xchg) a.xchg(a, ICE_GPU_HALO_CELLS);   // the remote source cells of the ghost layers
     if (a.ngrec + a.ncopy > 0) {
       const unsigned nrb = grid(a.ngrec, 128), g = nrb + GhostPart<CL>::n * grid(a.ncopy, 128);
@@ -72,9 +69,11 @@ void launch_family_t(const LaunchArgs& a) {
     }
     if (a.xchg) a.xchg(a, ICE_GPU_HALO_BETA);    // the weights of partner cells another rank steps
   }
-  if (a.part == PART_PREP) return;
-  launch_flux_of<CL>(a);
-  tick(a.plane ? KC_BOUND : KC_STAGE);         // (else the interior faces come with the records)
+  if (a.part & PART_FACES) {
+    launch_flux_of<CL>(a);
+    tick(a.plane ? KC_BOUND : KC_STAGE);         // (else the interior faces come with the records)
+  }
+  if (!(a.part & PART_CELLS)) return;
   if (!a.irs) {
     launch_stage_of<CL>(a, false);
     tick(KC_STAGE);

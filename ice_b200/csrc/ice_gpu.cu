@@ -156,7 +156,7 @@ struct ice_gpu_ctx {
   cudaStream_t s_up = nullptr, s_down = nullptr;
   // the step's second branch (capture_step), captured only
   cudaStream_t s_prep = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_prep[kMaxF] = {}, ev_done[kMaxF] = {};
+  cudaEvent_t ev_fork = nullptr, ev_prep[kMaxF] = {}, ev_done[kMaxF] = {}, ev_src[kMaxF] = {};
   cudaEvent_t ev_up = nullptr, ev_fam[kMaxF] = {};
   DevBuf<double> xall;
   int phase = 0;          // buffer holding the current state
@@ -248,6 +248,11 @@ static bool sur_active(const ice_gpu_ctx* c, int p);
 static bool sweeps64(const ice_gpu_ctx* c) { return c->P.precision != ICE_PREC_FP32FLUX || c->P.irs; }
 // The FP32-flux form's 1-D stage kernel runs (ice_kernels.cuh).
 static bool plane(const ice_gpu_ctx* c) { return !sweeps64(c) && c->P.ndir == 1; }
+
+// Family p's source has a kernel of its own.
+static bool own_source(const ice_gpu_ctx* c, int p) {
+  return c->P.coupled && (sweeps64(c) || plane(c) || sur_active(c, p) || c->P.fam[p].evap != 0);
+}
 
 // The buffer stage srk reads as its stencil (U_{k-1}) when the step starts from buffer `phase`.
 static int stencil_buffer(const ice_gpu_ctx*, int srk, int phase) {
@@ -468,6 +473,7 @@ static void launch_family(ice_gpu_ctx* c, int p, int srk, int phase, cudaStream_
   a.plane = plane(c);
   a.part = part;
   a.mlp_img = sur_active(c, p) ? H.mlp_img.p : nullptr;
+  a.own_source = own_source(c, p);
   a.mlp_norm = &H.mlp_norm;
   a.ndir = c->P.ndir; a.sd = c->P.shock_detector; a.irs = c->P.irs; a.precision = c->P.precision;
   a.irs_beta = c->P.irs_beta;
@@ -562,26 +568,36 @@ static void enqueue_step(ice_gpu_ctx* c, int phase, cudaStream_t s, void (*tick)
   for (int p = 0; p < c->P.nfam; ++p) enqueue_step_family(c, p, phase, s, tick);
 }
 
-// The step of several families as a graph of two branches: the families' faces and updates on s, stage by
-// stage, and on a second stream what comes before a family's faces (source, ghosts, sensor: kernels that wait
-// on memory or on their own chains), under the faces of the families before it. The families share the
-// face fluxes, so their faces stay one after the other. Three families on 8 blocks of 1.7 M cells, 8 steps in
-// the FP32-flux form 32.8 -> 31.4 ms; 4 blocks of 0.35 M cells, 5 steps in FP64 12.3 -> 11.5 ms.
+// The step as a graph of two branches: the families' faces and updates on s, stage by stage, and on a second
+// stream their ghosts and sensors, under the faces of the families before them, and their sources, which only
+// the update reads, under their own faces too: kernels that wait on memory or on their own chains beside
+// ones that leave half of the issue slots free. The families share the face fluxes, so their faces stay one
+// after the other. Three families on 8 blocks of 1.7 M cells, 8 steps in the FP32-flux form: 32.8 ms in one
+// branch, 31.4 in two; 4 blocks of 0.35 M cells, 5 steps in FP64: 12.3 and 11.5, 10.8 with the sources under the
+// faces. One family takes the second branch while a cell a thread is less than four waves: AG cells of 28 k
+// 1.83 / 1.69 ms (20 steps, FP32 form) and 261 k 8.47 / 8.35 (10 steps, FP64) gain, 885 k 9.88 / 10.04 lose.
+static bool two_branches(const ice_gpu_ctx* c) {
+  return c->P.nfam > 1 || (own_source(c, 0) && c->NI < 4LL * 4 * SW_NT * c->nsm);
+}
+
 static cudaError_t capture_step(ice_gpu_ctx* c, int phase, cudaStream_t s) {
-  const int nf = c->P.nfam;
-  if (nf < 2) { enqueue_step(c, phase, s, nullptr); return cudaSuccess; }
+  if (!two_branches(c)) { enqueue_step(c, phase, s, nullptr); return cudaSuccess; }
   cudaError_t e = cudaSuccess;
   auto ck = [&](cudaError_t x) { if (e == cudaSuccess) e = x; };
   enqueue_step_dt(c, phase, s, nullptr);
   ck(cudaEventRecord(c->ev_fork, s));
   ck(cudaStreamWaitEvent(c->s_prep, c->ev_fork, 0));
   for (int srk = 1; srk <= c->P.nrk; ++srk)
-    for (int p = 0; p < nf; ++p) {
+    for (int p = 0; p < c->P.nfam; ++p) {
       if (srk > 1) ck(cudaStreamWaitEvent(c->s_prep, c->ev_done[p], 0));
-      launch_family(c, p, srk, phase, c->s_prep, nullptr, PART_PREP);
+      launch_family(c, p, srk, phase, c->s_prep, nullptr, PART_GHOSTS);
       ck(cudaEventRecord(c->ev_prep[p], c->s_prep));
+      launch_family(c, p, srk, phase, c->s_prep, nullptr, PART_SOURCE);
+      ck(cudaEventRecord(c->ev_src[p], c->s_prep));
       ck(cudaStreamWaitEvent(s, c->ev_prep[p], 0));
       launch_family(c, p, srk, phase, s, nullptr, PART_FACES);
+      ck(cudaStreamWaitEvent(s, c->ev_src[p], 0));
+      launch_family(c, p, srk, phase, s, nullptr, PART_CELLS);
       ck(cudaEventRecord(c->ev_done[p], s));
     }
   return e;
@@ -590,12 +606,13 @@ static cudaError_t capture_step(ice_gpu_ctx* c, int phase, cudaStream_t s) {
 // The step's graph from buffer `phase`.
 static int step_graph(ice_gpu_ctx* c, int phase) {
   if (c->graph[phase]) return 0;
-  if (c->P.nfam > 1 && !c->s_prep) {
+  if (two_branches(c) && !c->s_prep) {
     CK(cudaStreamCreateWithFlags(&c->s_prep, cudaStreamNonBlocking));
     CK(cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
     for (int p = 0; p < c->P.nfam; ++p) {
       CK(cudaEventCreateWithFlags(&c->ev_prep[p], cudaEventDisableTiming));
       CK(cudaEventCreateWithFlags(&c->ev_done[p], cudaEventDisableTiming));
+      CK(cudaEventCreateWithFlags(&c->ev_src[p], cudaEventDisableTiming));
     }
   }
   cudaGraph_t g;
@@ -625,8 +642,7 @@ static long long launches_per_step(const ice_gpu_ctx* c) {
   for (int p = 0; p < c->P.nfam; ++p) n += c->fam[p].have_imp ? 3 : 0;
   for (int p = 0; p < c->P.nfam; ++p) {
     const FamHost& H = c->fam[p];
-    const bool own_source = c->P.coupled && (sweeps64(c) || plane(c) || sur_active(c, p) || c->P.fam[p].evap != 0);
-    long long per = (H.ngrec + H.ncopy > 0 ? (H.ghost_split ? 2 : 1) : 0) + (c->P.shock_detector ? 1 : 0) + (own_source ? 1 : 0) +
+    long long per = (H.ngrec + H.ncopy > 0 ? (H.ghost_split ? 2 : 1) : 0) + (c->P.shock_detector ? 1 : 0) + (own_source(c, p) ? 1 : 0) +
                     (H.nfrec + H.nzface > 0 || (!plane(c) && H.nfjob > 0));
     per += c->P.irs ? (2 + 2 * c->P.ndir) : 1;
     n += per * c->P.nrk;
@@ -893,6 +909,7 @@ int ice_gpu_destroy(ice_gpu_ctx* c) {
   if (c->ev_fork) cudaEventDestroy(c->ev_fork);
   for (auto& e : c->ev_prep) if (e) cudaEventDestroy(e);
   for (auto& e : c->ev_done) if (e) cudaEventDestroy(e);
+  for (auto& e : c->ev_src) if (e) cudaEventDestroy(e);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;
   return 0;

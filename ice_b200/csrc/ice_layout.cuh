@@ -150,9 +150,8 @@ enum { SW_X = 0, SW_Y = 1, SW_Z = 2 };
 struct SweepJob { int b, kind, base, c0, n; };
 struct NormChunk { int b; long long q0, q1; };
 
-// The parts of a family's stage: what comes before its faces (source, ghosts, sensor), and the faces and the
-// update.
-enum { PART_ALL = 0, PART_PREP, PART_FACES };
+// The parts of a family's stage: its source's own kernel, its ghosts and sensor, its faces, its cells' update.
+enum { PART_SOURCE = 1, PART_GHOSTS = 2, PART_FACES = 4, PART_CELLS = 8, PART_ALL = 15 };
 
 // Everything one family's stage needs, for the launcher of its closure's translation unit.
 struct LaunchArgs {
@@ -165,10 +164,11 @@ struct LaunchArgs {
   const int* frec; int nfrec;                        // the records whose flux is computed, in thread order
   const SweepJob* fjobs; int nfjob;                  // the flux kernel's CTAs
   const Tile* tiles; int ntile; int TX, TY, KZ;     // the 1-D stage kernel's tiles
+  bool own_source;                                   // the source has a kernel of its own
   const unsigned char* mlp_img;                      // the family's surrogate network (null: the plain closure)
   const MlpNorm* mlp_norm;
   int ndir, sd, irs, precision;
-  int part;                                          // PART_*
+  int part;                                          // PART_* bits
   int plane;                                         // the FP32-flux form's 1-D stage kernel runs (ice_kernels.cuh)
   double irs_beta;
   double* resid; double* resid2; double* resid3;
