@@ -70,6 +70,17 @@ template <typename T> struct DevBuf {
     if (count == 0) return cudaSuccess;
     return cudaMalloc((void**)&p, count * sizeof(T));
   }
+  // For what a run could do without at a price: where the device has no room left, managed memory, whose pages
+  // lie on the host until they are used.
+  cudaError_t alloc_or_managed(size_t count) {
+    cudaError_t e = alloc(count);
+    if (e != cudaErrorMemoryAllocation) return e;
+    cudaGetLastError();
+    p = nullptr;
+    e = cudaMallocManaged((void**)&p, count * sizeof(T));
+    if (e != cudaSuccess) { p = nullptr; n = 0; }
+    return e;
+  }
 };
 
 struct FamHost {
@@ -120,7 +131,7 @@ struct ice_gpu_ctx {
   long long NG = 0, NI = 0, NR = 0, NF[3] = {0, 0, 0};
   DevBuf<DBlock> blk;
   DevBuf<double> face[3], vol, dl, M, gas;
-  DevBuf<double> row;       // Geo::row, formed from M with each block's metrics
+  DevBuf<double> row;       // Geo::row, formed from M before the first step after a block's metrics
   DevBuf<float4> facef[3];  // the FP32-flux form's geometry (Geo::ff, dlf), rounded from the FP64 arrays
   DevBuf<float> dlf;
   DevBuf<float> gasf;       // the FP32-flux form's copy of the gas (Geo::gasf)
@@ -129,7 +140,7 @@ struct ice_gpu_ctx {
   DevBuf<unsigned char> flux;
   size_t flux_at[3] = {0, 0, 0};
   int flux_word = 0;
-  bool flux_ok = false;
+  bool flux_ok = false, rows_ok = false;
   bool geo32_ok = false;
   bool have_gas = false;
   std::vector<bool> have_block;
@@ -744,9 +755,18 @@ static int build_sweeps(ice_gpu_ctx* c) {
   return 0;
 }
 
-// The face fluxes: the largest family's, in the word of the running form; the faces no record gives a flux are
-// zero and stay so. Before the first step, after a change of form, after a new boundary table.
+// What a step keeps beyond its states and inputs: the metric rows (after a block's metrics) and the face fluxes,
+// the largest family's, in the word of the running form; the faces no record gives a flux are zero and stay so
+// (before the first step, after a change of form, after a new boundary table). 96 + 12 nc (24 nc) bytes a cell
+// in 3-D, allocated last and, on a device that the rest fills, in managed memory: such a run is slower, not
+// refused.
 static int ensure_flux(ice_gpu_ctx* c) {
+  if (!c->rows_ok) {
+    if (!c->row.p) CK(c->row.alloc_or_managed((size_t)12 * c->NI));
+    k_rows<<<grid_of(c->NI), 256, 0, c->stream>>>(c->M.p, c->row.p, c->NI, 0, c->NI);
+    CK(cudaGetLastError());
+    c->rows_ok = true;
+  }
   const int word = sweeps64(c) ? 8 : 4;
   if (c->flux_ok && c->flux_word == word) return 0;
   size_t nc = 0;
@@ -758,11 +778,14 @@ static int ensure_flux(ice_gpu_ctx* c) {
     c->flux_at[d] = n;
     n += (nc * c->NF[d] * word + 255) & ~(size_t)255;
   }
-  if (c->flux_word != word) CK(c->flux.alloc(n));
+  if (c->flux_word != word) {
+    c->flux_word = 0;
+    CK(c->flux.alloc_or_managed(n));
+  }
   CK(cudaMemsetAsync(c->flux.p, 0, n, c->stream));
   for (int p = 0; p < c->P.nfam; ++p)
     if (word == 4 && c->P.shock_detector && !c->fam[p].betaf.p) {
-      CK(c->fam[p].betaf.alloc(c->NI));
+      CK(c->fam[p].betaf.alloc_or_managed(c->NI));
       free_graphs(c);
     }
   c->flux_word = word;
@@ -857,7 +880,6 @@ int ice_gpu_create(const ice_gpu_params* P, int32_t nblocks, const int32_t* dims
   CKC(c->vol.alloc(I));
   CKC(c->dl.alloc((size_t)3 * R));
   CKC(c->M.alloc((size_t)9 * I));
-  CKC(c->row.alloc((size_t)12 * I));
   if (P->coupled) CKC(c->gas.alloc((size_t)9 * I));
   for (int p = 0; p < P->nfam; ++p) {
     FamHost& H = c->fam[p];
@@ -956,10 +978,9 @@ int ice_gpu_set_block(ice_gpu_ctx* c, int32_t b1, const double* f1, const double
     CK(cudaMemcpy(c->M.p + (long long)comp * c->NI + B.ioff, tmp.data(), ncell * sizeof(double), cudaMemcpyHostToDevice));
   }
   CK(cudaStreamSynchronize(c->stream));
-  k_rows<<<grid_of(ncell), 256, 0, c->stream>>>(c->M.p, c->row.p, c->NI, B.ioff, ncell);
-  CK(cudaGetLastError());
   c->have_block[b1 - 1] = true;
   c->geo32_ok = false;
+  c->rows_ok = false;
   return 0;
 }
 
@@ -1560,7 +1581,6 @@ int ice_gpu_step_host(ice_gpu_ctx* c, int32_t nsteps, const double* const* prim_
   if (!c) return ICE_GPU_EINVAL;
   if (int rc = check_ready(c)) return rc;
   if (int rc = build_geo32(c)) return rc;
-  if (int rc = ensure_flux(c)) return rc;
   if (nsteps < 1) return fail(c, ICE_GPU_EINVAL, "step_host: nsteps %d", nsteps);
   if (!prim_in || !prim_out) return fail(c, ICE_GPU_EINVAL, "step_host: null array list");
   if (!c->owned.empty()) return fail(c, ICE_GPU_EINVAL, "step_host: a split run steps through ice_gpu_step");
@@ -1588,6 +1608,7 @@ int ice_gpu_step_host(ice_gpu_ctx* c, int32_t nsteps, const double* const* prim_
     for (int p = 0; p < nf; ++p) off[(size_t)b * nf + p + 1] = off[(size_t)b * nf + p] + ng * c->fam[p].nc;
   }
   if (c->xall.n < (size_t)off.back()) CK(c->xall.alloc((size_t)off.back()));
+  if (int rc = ensure_flux(c)) return rc;        // after xall: the fluxes can do without device memory
   if (!c->s_up) CK(cudaStreamCreateWithFlags(&c->s_up, cudaStreamNonBlocking));
   if (!c->s_down) CK(cudaStreamCreateWithFlags(&c->s_down, cudaStreamNonBlocking));
   if (!c->ev_up) CK(cudaEventCreateWithFlags(&c->ev_up, cudaEventDisableTiming));

@@ -20,9 +20,9 @@
 // 128 registers or fewer and no barrier, every direction is in flight at once, and the fluxes cost
 // 6 nc words per cell of bandwidth that stood idle. FP64: the two divisions of every limited slope
 // run branchless and side by side (ice_div.h), where a compiled division's branch ordered them one after the
-// other. Stage kernels, per launch pair, old / new (one B200, CUDA events): FP64 IG 96 x 95 x 97 967 / 303 us,
-// AG 64 x 61 x 67 693 + 161 (records) / 217 us; FP32 form IG 128 x 126 x 129 516 + 28 / 352 us,
-// AG 96^3 387 + 30 / 284 us.
+// other. Stage kernels, the one kernel (+ records) / k_flux + k_cells (one B200, CUDA events): FP64 IG
+// 96 x 95 x 97 967 / 212 + 74 us, AG 64 x 61 x 67 693 + 161 / 146 + 49 us; FP32 form IG 128 x 126 x 129
+// 516 + 28 / 173 + 139 us, AG 96^3 387 + 30 / 152 + 105 us.
 #pragma once
 #include "ice_kernels.cuh"
 
@@ -31,13 +31,19 @@ namespace ice {
 constexpr int SW_NT = 128;                      // threads per CTA
 constexpr int SW_XC = SW_NT / 32 * 31;          // cells whose upper x face one CTA computes
 
-// The CTAs per SM the flux and the cell kernel are held to. Flux: 6 against 5 in the FP32-flux form 192 / 214 us
-// (IG, 128 x 126 x 129; AG at 6 spills, 209 / 164 us on 96^3), 3 against 2 for FP64 AG 152 / 160 us
-// (64 x 61 x 67), 4 against 3 and 5 for FP64 IG 225 / 248 / 246 us (96 x 95 x 97). Cells: 5 against 6 139 / 145 us
-// (FP32 IG), AG 2 against 3 56 / 69 us (FP64): its loads are what it holds registers for.
+// The CTAs per SM the flux and the cell kernel are held to, and which loads of the cell kernel wait.
+// Flux: 6 against 5 in the FP32-flux form 192 / 214 us (IG, 128 x 126 x 129; AG at 6 spills, 209 / 164 us on
+// 96^3), 3 against 2 for FP64 AG 152 / 160 us (64 x 61 x 67), 4 against 3 and 5 for FP64 IG 225 / 248 / 246 us
+// (96 x 95 x 97).
+// Cells: a warp holds a register for every load in flight, so a cell's six fluxes and its state at once cost
+// warps. late 1 asks for the state only when the x and y fluxes are summed, 2 for the z fluxes too. AG FP64:
+// 56.5 us with all at once at 2 CTAs, 56.0 / 57.3 at late 1 and 2, 48.3 - 50.1 at late 2 and 3 CTAs (all at
+// once and 3 CTAs: 69, it spills). AG FP32 (4 CTAs): 126.8 us all at once, 104.7 at late 1, 109.0 at late 2. IG FP64 (4):
+// 77.3 / 73.7 / 81.3 us at late 0, 1, 2. IG FP32 (5): 139.5 / 145.4 / 154.0: there all at once is best.
 template <int CL, typename R> struct SweepOcc {
   static constexpr int flux = sizeof(R) == 8 ? (CL == AG ? 3 : 4) : (CL == AG ? 4 : 6);
-  static constexpr int cells = sizeof(R) == 8 ? (CL == AG ? 2 : 4) : (CL == AG ? 4 : 5);
+  static constexpr int cells = sizeof(R) == 8 ? (CL == AG ? 3 : 4) : (CL == AG ? 4 : 5);
+  static constexpr int late = sizeof(R) == 8 ? (CL == AG ? 2 : 1) : (CL == AG ? 1 : 0);
 };
 
 // Limited slope of one cell from its two difference quotients.
@@ -350,19 +356,20 @@ __global__ void __launch_bounds__(SW_NT, SweepOcc<CL, R>::cells) k_cells(Geo G, 
   const unsigned jk = l / ni;
   const int i = (int)(l % ni), j = (int)(jk % nj), k = (int)(jk / nj);
   const long long g = gidx(B, i, j, k);
+  constexpr int LATE = SweepOcc<CL, R>::late;
   double p[nc];
   R x0[nc], x1[nc], y0[nc], y1[nc], z0[nc], z1[nc];
-  {                                              // every flux of the cell on its way before the first use
+  const R* z = (const R*)F.Ff[2] + fidx(B, 2, i, j, k, k);
+  const long long up = (long long)B.ni * B.nj;
+  {                                              // on their way before the first use
     const R* x = (const R*)F.Ff[0] + fidx(B, 0, i, j, k, i);
     const R* y = (const R*)F.Ff[1] + fidx(B, 1, i, j, k, j);
-    const R* z = (const R*)F.Ff[2] + fidx(B, 2, i, j, k, k);
-    const long long up = (long long)B.ni * B.nj;
 #pragma unroll
     for (int v = 0; v < nc; ++v) {
       x0[v] = x[v * G.NF[0]]; x1[v] = x[v * G.NF[0] + 1];
       y0[v] = y[v * G.NF[1]]; y1[v] = y[v * G.NF[1] + B.ni];
-      z0[v] = z[v * G.NF[2]]; z1[v] = z[v * G.NF[2] + up];
-      p[v] = F.Up[(long long)v * G.NG + g];
+      if (LATE < 2) { z0[v] = z[v * G.NF[2]]; z1[v] = z[v * G.NF[2] + up]; }
+      if (LATE < 1) p[v] = F.Up[(long long)v * G.NG + g];
     }
   }
   R r[nc];
@@ -370,13 +377,21 @@ __global__ void __launch_bounds__(SW_NT, SweepOcc<CL, R>::cells) k_cells(Geo G, 
   for (int v = 0; v < nc; ++v) r[v] = (R)0;
   if (i == 0 || i == B.ni - 1 || j == 0 || j == B.nj - 1 || k == 0 || k == B.nk - 1) {
     double acc[nc];
-    edge_sum<nc>(B, i, j, k, acc, [&](int d, int v) { return d == 0 ? x0[v] : d == 1 ? y0[v] : z0[v]; },
-                 [&](int d, int v) { return d == 0 ? x1[v] : d == 1 ? y1[v] : z1[v]; });
+    edge_sum<nc>(B, i, j, k, acc, [&](int d, int v) { return d == 0 ? x0[v] : d == 1 ? y0[v] : LATE < 2 ? z0[v] : z[v * G.NF[2]]; },
+                 [&](int d, int v) { return d == 0 ? x1[v] : d == 1 ? y1[v] : LATE < 2 ? z1[v] : z[v * G.NF[2] + up]; });
 #pragma unroll
     for (int v = 0; v < nc; ++v) r[v] = (R)acc[v];
   }
   if (B.ni >= 2) add_faces<nc>(r, i + 1, B.ni, x0, x1);
   if (B.nj >= 2) add_faces<nc>(r, j + 1, B.nj, y0, y1);
+  if constexpr (LATE > 0) {
+    asm volatile("" ::: "memory");               // keeps these loads behind the sums above
+#pragma unroll
+    for (int v = 0; v < nc; ++v) {
+      if (LATE > 1) { z0[v] = z[v * G.NF[2]]; z1[v] = z[v * G.NF[2] + up]; }
+      p[v] = F.Up[(long long)v * G.NG + g];
+    }
+  }
   if (B.nk >= 2) add_faces<nc>(r, k + 1, B.nk, z0, z1);
   cell_update<CL, R>(G, F, q, g, r, p, write_r, st);
 }
