@@ -94,7 +94,7 @@ def algorithmic_bytes(case, precision: int = abi.PREC_FP64) -> float:
     form) and the relaxation time it writes on the last stage (8 / nrk), or, for an evaporating family
     of a 2-D or 3-D run, the source its own kernel wrote (8 nc; 4 nc in single precision in the FP32-flux
     form); the local dt (8) in steady mode; in 1-D runs the sensor weight (8) when the shock detector
-    is on (2-D and 3-D runs evaluate it from the staged density)."""
+    is on."""
     ndir = case.ndir
     nrk = case.params().nrk
     per = []
