@@ -39,11 +39,14 @@ constexpr int SW_XC = SW_NT / 32 * 31;          // cells whose upper x face one 
 // warps. late 1 asks for the state only when the x and y fluxes are summed, 2 for the z fluxes too. AG FP64:
 // 56.5 us with all at once at 2 CTAs, 56.0 / 57.3 at late 1 and 2, 48.3 - 50.1 at late 2 and 3 CTAs (all at
 // once and 3 CTAs: 69, it spills). AG FP32 (4 CTAs): 126.8 us all at once, 104.7 at late 1, 109.0 at late 2. IG FP64 (4):
-// 77.3 / 73.7 / 81.3 us at late 0, 1, 2. IG FP32 (5): 139.5 / 145.4 / 154.0: there all at once is best.
+// 77.3 / 73.7 / 81.3 us at late 0, 1, 2. IG FP32: 138.9 us all at once at 5 CTAs, 136.8
+// at late 1 and 6 (145.4 and 144.5 with one of the two). MK FP32: flux 7 against 6 and cells 6 against 5, all at
+// once, with IG's: three families on 8 blocks, 1.7 M cells, 29.3 -> 28.6 ms of 8 steps, flux 202 -> 199 us and
+// cells 138 -> 134 (means of the families).
 template <int CL, typename R> struct SweepOcc {
-  static constexpr int flux = sizeof(R) == 8 ? (CL == AG ? 3 : 4) : (CL == AG ? 4 : 6);
-  static constexpr int cells = sizeof(R) == 8 ? (CL == AG ? 3 : 4) : (CL == AG ? 4 : 5);
-  static constexpr int late = sizeof(R) == 8 ? (CL == AG ? 2 : 1) : (CL == AG ? 1 : 0);
+  static constexpr int flux = sizeof(R) == 8 ? (CL == AG ? 3 : 4) : CL == AG ? 4 : CL == IG ? 6 : 7;
+  static constexpr int cells = sizeof(R) == 8 ? (CL == AG ? 3 : 4) : CL == AG ? 4 : 6;
+  static constexpr int late = sizeof(R) == 8 ? (CL == AG ? 2 : 1) : CL == MK ? 0 : 1;
 };
 
 // Limited slope of one cell from its two difference quotients.
