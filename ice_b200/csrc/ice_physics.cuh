@@ -504,7 +504,7 @@ __device__ __forceinline__ void limited(int lim, const R* x, const R* y, R cx, R
   } else {
     const int kind = LIM == LIM_ANY ? lim : LIM;
     R ru[nc], phi[nc];
-    unsigned low = 0;                // the largest low word of a divisor (all ones: ice_div_by)
+    unsigned low = 0;                // the largest low word of a divisor (ice_div_by)
 #pragma unroll
     for (int v = 0; v < nc; ++v) {
       const R d = x[v] + (R)1e-30;
@@ -540,7 +540,7 @@ __device__ __forceinline__ void limited(int lim, const R* x, const R* y, R cx, R
       if (LIM == ICE_LIM_VANLEER || (kind != ICE_LIM_MINMOD && ru[v] > (R)0)) phi[v] = mn(mn(phi[v], cx), cy*ru[v]);
       s[v] = first ? (R)0 : phi[v] * x[v];
     }
-    if ((!fast || low == 0xffffffffu) && !first) {
+    if ((!fast || low >= ICE_DIV_LOW) && !first) {
 #pragma unroll
       for (int v = 0; v < nc; ++v) s[v] = limiter_any(kind, x[v], y[v], cx, cy);
     }

@@ -9,13 +9,22 @@
  * keep every intermediate value normal. ice_div_in and ice_div_by say whether they do; the caller
  * divides with `/` otherwise. The result is then the IEEE quotient, bit for bit (a zero dividend gives +0 or -0).
  *
- * Why it is the IEEE quotient: let m in [1, 2) be the significand of b. recip's last step leaves y within
- * (1/2 + 2^-24) ulp of 1/b, a relative error of 2^-54 m. quot's first correction leaves q within
- * (1/2 + 2^-50) ulp of a/b; its remainder a - b q is exact. The last step rounds q + r y, which is a/b
- * moved by at most 2^-55 m ulp, while a/b is at least 2^-53 / m ulp from any midpoint of two doubles: the
- * move is the smaller for every m but those next to 2, of which only the largest, all ones, is rounded
- * wrongly (for powers of two above it). ice_div_by excludes it. tests/test_div.py checks the rest against
- * `/`, significands next to 1 and 2 included.
+ * Why it is the IEEE quotient: let m = 2 - j 2^-52 in [1, 2) be the significand of b and e0 the relative error of the
+ * first approximation: on one B200 2^-19.93 at most over every upper word, 2^-21 where the upper twenty bits of the
+ * significand are ones (j <= 2^32). Two Newton steps leave e0^4, below 2^-79.6 and for j <= 2^32 below 2^-79.9 (from
+ * 2^-20 on), and the last rounding: y = (1 + t) / b, |t| <= 2^-54 m + e0^4, half an ulp of 1/b (whose significand is 2 / m)
+ * and the rest.
+ * quot's first correction leaves q within (1/2 + 2^-50) ulp of a/b, so its remainder a - b q is exact. The last step
+ * rounds q + r y: a/b moved by at most (1/2 + 2^-50) |t| ulp. A quotient of two doubles is at least 2^-53 / m ulp
+ * from any midpoint, which leaves 2^-55 (4 - m^2) / m >= j 2^-106 ulp for t beyond 2^-54 m and for the 2^-50.
+ *   j > 2^32: 2^-74 and more is left, 2^-80.6 + 2^-103 taken.
+ *   2^26 < j <= 2^32: 2^-80 and more is left, 2^-80.9 + 2^-103 taken.
+ *   2^14 < j <= 2^26: 1/b has the significand 1 + j h + j^2 h^2 + ..., h = 2^-53, ulp 2 h: for odd j it lies j^2 h^2 > 2^-78
+ *     above a tie of doubles, for even j more than 2^-55 off one, so y is 1/b rounded correctly and t has no rest; 2^-92 and
+ *     more is left, 2^-103 taken.
+ *   j <= 2^14: y may fall on the other side of its tie, and some quotients next to a midpoint are then rounded
+ *     wrongly. ice_div_by excludes them by the low word, of every divisor.
+ * tests/test_div.py and tests/test_div_midpoints.py check it against `/`.
  */
 #ifndef ICE_DIV_H
 #define ICE_DIV_H
@@ -41,7 +50,10 @@ ICE_DIV_FN unsigned ice_div_hi(double x) {
 /* 2^-200 <= |x| < 2^200: x is a dividend of the quotients below (and zero is one). */
 ICE_DIV_FN int ice_div_in(double x) { return ice_div_hi(x) - (823u << 20) < (400u << 20); }
 
-/* x is a divisor of the quotients below: the same range, and its low word is not all ones. */
+/* The low words that no divisor has (see above). */
+#define ICE_DIV_LOW 0xffffc000u
+
+/* x is a divisor of the quotients below: the same range, and its low word is below ICE_DIV_LOW. */
 ICE_DIV_FN int ice_div_by(double x) {
 #ifdef __CUDA_ARCH__
   const unsigned lo = (unsigned)__double2loint(x);
@@ -50,10 +62,10 @@ ICE_DIV_FN int ice_div_by(double x) {
   v.d = x;
   const unsigned lo = (unsigned)v.u;
 #endif
-  return ice_div_in(x) && lo != 0xffffffffu;
+  return ice_div_in(x) && lo < ICE_DIV_LOW;
 }
 
-/* The first approximation of 1/b, good to 2^-20 or better (rcp.approx.ftz.f64 on the device). */
+/* The first approximation of 1/b (rcp.approx.ftz.f64 on the device; its error: see above). */
 ICE_DIV_FN double ice_div_seed(double b) {
 #ifdef __CUDA_ARCH__
   double y;
