@@ -29,7 +29,7 @@ template <int CL> inline void launch_beta_of(const LaunchArgs& a) {
 }
 
 template <int CL> inline void launch_source_of(const LaunchArgs& a) {
-  const bool f32 = a.precision == ICE_PREC_FP32FLUX;
+  const bool f32 = a.precision == ICE_PREC_FP32FLUX && !a.irs;
   if constexpr (CL == MK) { if (f32) launch_source_mk_f32(a); else launch_source_mk_f64(a); }
   else if constexpr (CL == IG) { if (f32) launch_source_ig_f32(a); else launch_source_ig_f64(a); }
   else { if (f32) launch_source_ag_f32(a); else launch_source_ag_f64(a); }

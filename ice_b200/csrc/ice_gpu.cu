@@ -301,7 +301,7 @@ static FamDev make_famdev(ice_gpu_ctx* c, int p, int srk, int phase) {
   F.dtg = &c->st.p->dtglobal;
   F.tau = H.tau.p;
   F.S = H.src.p;
-  F.Sf = c->P.precision == ICE_PREC_FP32FLUX ? (float*)H.src.p : nullptr;
+  F.Sf = sweeps64(c) ? nullptr : (float*)H.src.p;      // an IRS run's stage, and so its source, is FP64 in both forms
   F.connF = c->owned.empty() ? nullptr : H.connF.p;
   for (int d = 0; d < 3; ++d) F.Ff[d] = c->flux.p + c->flux_at[d];
   F.zface = H.zface.p; F.nzface = H.nzface;
