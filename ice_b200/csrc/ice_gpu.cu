@@ -1222,9 +1222,9 @@ int ice_gpu_set_records(ice_gpu_ctx* c, int32_t nrec, const int32_t* ri, const d
       d.owner = r.owner; d.cf = r.cf - 1;
       if (r.type == 101 || r.type == 201) {
         const HRec& q2 = c->recs[r.partner - 1];
-        d.pb = q2.b - 1; d.pi = q2.i - 1; d.pj = q2.j - 1; d.pk = q2.k - 1;
+        d.pb = q2.b - 1; d.pi = q2.i - 1; d.pj = q2.j - 1; d.pk = q2.k - 1; d.pf = q2.f;
         ncf = std::max(ncf, r.cf);
-      } else { d.pb = d.pi = d.pj = d.pk = 0; }
+      } else { d.pb = d.pi = d.pj = d.pk = 0; d.pf = 1; }
       d.normal_dir = r.normal_dir != 0.0;
       d.massflux = r.massflux; d.velocity = r.velocity; d.alpha = r.alpha; d.beta = r.beta;
       d.temperature = r.temperature; d.radius = r.radius; d.gfixed = r.gfixed;

@@ -742,7 +742,7 @@ __device__ __forceinline__ bool rec_face(const Geo& G, const FamDev& F, const DR
   }
   put_flux<CL, R>(G, F, G.blk[r.b], r.f, r.i, r.j, r.k, fl, 1.0);
   if (conn) {
-    put_flux<CL, R>(G, F, G.blk[r.pb], r.fs, r.pi, r.pj, r.pk, fl, -1.0);
+    put_flux<CL, R>(G, F, G.blk[r.pb], r.pf, r.pi, r.pj, r.pk, fl, -1.0);
     if (F.connF) {
 #pragma unroll
       for (int v = 0; v < nc; ++v) F.connF[(long long)r.cf * nc + v] = fl[v];

@@ -45,7 +45,7 @@ struct DRec {                // one boundary record, 0-based cells
   int bs, is, js, ks, fs;
   int owner, cf;             // cf 0-based (-1 when none)
   int next;                  // another record of the same cell and face (place in the family's records), or -1
-  int pb, pi, pj, pk;        // the partner's cell (connections)
+  int pb, pi, pj, pk, pf;    // the partner's cell and its own face (connections; fs says where the ghosts come from)
   int normal_dir;
   double massflux, velocity, alpha, beta, temperature, radius, gfixed;
   // host-computed once per record (the platform libm of the driver's host, as the
