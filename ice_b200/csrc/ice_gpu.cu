@@ -101,6 +101,8 @@ struct FamHost {
   bool ghost_split = false;                  // the ghost layers in two launches (upload_recs)
   DevBuf<int> frec;                          // the records whose flux is computed, in the record kernel's thread order
   int nfrec = 0;
+  DevBuf<int> sfirst, slist;                 // the cells of k_cell_sum: their first records, their records
+  int nsum = 0;
   DevBuf<ZeroFace> zface;                    // FamDev::zface
   int nzface = 0;
   DevBuf<SweepJob> fjobs;                    // the flux kernel's CTAs (ice_sweep.cuh)
@@ -302,7 +304,7 @@ static FamDev make_famdev(ice_gpu_ctx* c, int p, int srk, int phase) {
   F.tau = H.tau.p;
   F.S = H.src.p;
   F.Sf = sweeps64(c) ? nullptr : (float*)H.src.p;      // an IRS run's stage, and so its source, is FP64 in both forms
-  F.connF = c->owned.empty() ? nullptr : H.connF.p;
+  F.connF = c->owned.empty() && H.nsum == 0 ? nullptr : H.connF.p;
   for (int d = 0; d < 3; ++d) F.Ff[d] = c->flux.p + c->flux_at[d];
   F.zface = H.zface.p; F.nzface = H.nzface;
   F.cdon = H.cdon.p; F.cw = H.cw.p;
@@ -484,6 +486,7 @@ static void launch_family(ice_gpu_ctx* c, int p, int srk, int phase, cudaStream_
   a.grecs = H.grecs.p; a.ngrec = H.ngrec; a.gcopy = H.gcopy.p; a.ncopy = H.ncopy; a.next = H.next;
   a.frec = H.frec.p; a.nfrec = H.nfrec;
   a.fjobs = H.fjobs.p; a.nfjob = H.nfjob;
+  a.sfirst = H.sfirst.p; a.slist = H.slist.p; a.nsum = H.nsum;
   a.tiles = c->tiles.p; a.ntile = c->ntile; a.TX = c->TX; a.TY = c->TY; a.KZ = c->KZ;
   a.plane = plane(c);
   a.part = part;
@@ -658,7 +661,7 @@ static long long launches_per_step(const ice_gpu_ctx* c) {
   for (int p = 0; p < c->P.nfam; ++p) {
     const FamHost& H = c->fam[p];
     long long per = (H.ngrec + H.ncopy > 0 ? (H.ghost_split ? 2 : 1) : 0) + (c->P.shock_detector ? 1 : 0) + (own_source(c, p) ? 1 : 0) +
-                    (H.nfrec + H.nzface > 0 || (!plane(c) && H.nfjob > 0));
+                    (H.nfrec + H.nzface > 0 || (!plane(c) && H.nfjob > 0)) + (H.nsum > 0);
     per += c->P.irs ? (2 + 2 * c->P.ndir) : 1;
     n += per * c->P.nrk;
   }
@@ -1098,8 +1101,9 @@ int ice_gpu_update_params(ice_gpu_ctx* c, const ice_gpu_params* P) {
 
 // The family's device records (table order, which the record kernel indexes), and what the ghost kernel
 // reads, ordered by block, face and cell with the first index fastest, so that the threads of a warp fill
-// neighbouring ghost cells of one face (a record's ghosts are its own, so the order of the fills does not
-// change a value): the copying records of the stepped blocks as GhostCopy, the others as they are.
+// neighbouring ghost cells of one face (a face's ghosts are its own, so the order of the fills does not
+// change a value): the copying records of the stepped blocks as GhostCopy, the others as they are, and the records of a face
+// listed more than once one after the other in table order, for one thread.
 // ghost_split: some record's block (or, for a connection, its source block) is one cell deep along the
 // record's face direction, so that record's second ghost layer reads the first layer of the opposite face's
 // record; the ghost kernel then runs as two launches, every record as it is.
@@ -1131,10 +1135,18 @@ static int upload_recs(ice_gpu_ctx* c, FamHost& H) {
   };
   std::vector<DRec> g;
   std::vector<GhostCopy> ext, copy;
-  for (int q : ord) {
-    const DRec& r = dr[q];
+  auto same = [&](size_t x, size_t y) {
+    const DRec& a = dr[ord[x]]; const DRec& b = dr[ord[y]];
+    return a.b == b.b && a.f == b.f && a.k == b.k && a.j == b.j && a.i == b.i;
+  };
+  size_t end = 0;                                            // of the records of one face
+  for (size_t n = 0; n < ord.size(); ++n) {
+    const bool lead = n == end;
+    if (lead) while (end < ord.size() && same(n, end)) ++end;
+    DRec r = dr[ord[n]];
+    r.run = lead ? (int)(end - n) : 0;
     const bool conn = r.type == 101 || r.type == 201;
-    if (H.ghost_split || !(conn || r.type == 0 || r.type == 400)) { g.push_back(r); continue; }
+    if (H.ghost_split || r.run != 1 || !(conn || r.type == 0 || r.type == 400)) { g.push_back(r); continue; }
     if (!c->owned.empty() && !c->owned[r.b]) continue;       // a split run fills its own blocks' ghosts
     const int g0 = (r.f == 1) - (r.f == 2), g1 = (r.f == 3) - (r.f == 4), g2 = (r.f == 5) - (r.f == 6);
     GhostCopy x;
@@ -1205,6 +1217,7 @@ int ice_gpu_set_records(ice_gpu_ctx* c, int32_t nrec, const int32_t* ri, const d
     if ((t == 401 || t == 403) && r.massflux != 0.0 && !c->P.coupled)
       return fail(c, ICE_GPU_EINVAL, "record %d: inlet %d takes its speed from the gas, and the run has no gas", n + 1, t);
   }
+  std::vector<std::vector<int>> sum_cells(c->P.nfam);     // per family, a record of each cell of k_cell_sum
   for (int p = 0; p < c->P.nfam; ++p) {
     FamHost& H = c->fam[p];
     // the family's records in table order
@@ -1231,7 +1244,7 @@ int ice_gpu_set_records(ice_gpu_ctx* c, int32_t nrec, const int32_t* ri, const d
       d.ca = cos(r.alpha); d.sa = sin(r.alpha); d.cb = cos(r.beta); d.sb = sin(r.beta);
       d.vol_p = 4.0/3.0*kPi*pow(r.radius, 3.0);
       d.cd0 = d.cn1 = d.cn2 = 0;
-      d.next = -1;
+      d.run = 1; d.summed = 0;
     }
     H.nrec = (int)grp.size();
     H.h_grp = grp;
@@ -1271,22 +1284,49 @@ int ice_gpu_set_records(ice_gpu_ctx* c, int32_t nrec, const int32_t* ri, const d
     }
     H.nown = (int)H.h_own.size();
     H.ncf = ncf;
-    // the records whose flux is computed: connections by their owner; the symmetry records (200) of an MK family
-    // carry none (Mod_BC_Fluxes.f90:128). A face listed twice: its later records follow the first (DRec::next).
+    // the records whose flux is computed: connections by their owner (of several with one number the last, as
+    // one after the other would leave it); the symmetry records (200) of an MK family carry none (Mod_BC_Fluxes.f90:128)
     auto has_flux = [&](const DRec& d) { return d.type != 0 && !(d.type == 200 && H.closure == ICE_CLOSURE_MK); };
-    std::vector<int> fr;
+    auto is_conn = [](const DRec& d) { return d.type == 101 || d.type == 201; };
+    std::vector<int> giver(ncf, -1);
+    for (size_t q = 0; q < grp.size(); ++q)
+      if (is_conn(H.h_recs[q]) && H.h_recs[q].owner) giver[H.h_recs[q].cf] = (int)q;
+    // the place of x's partner among the family's records where x's flux is the partner's too, or -1
+    auto taker = [&](int x) {
+      const int y = pos[c->recs[grp[x]].partner - 1];
+      return y >= 0 && is_conn(H.h_recs[y]) && !H.h_recs[y].owner && H.h_recs[y].cf == H.h_recs[x].cf ? y : -1;
+    };
+    for (int x : giver) if (x >= 0 && taker(x) < 0) H.h_recs[x].pf = 0;
+    // the cells whose fluxes k_cell_sum adds: a face listed more than once, a connection that takes its number's flux otherwise
+    std::vector<int> fr, sfirst, slist;
     for (size_t q = 0; q + 1 < H.h_first.size(); ++q) {
-      int last = -1;
+      bool sum = false;
+      int face = 0;
+      const size_t at = slist.size(), fat = fr.size();
       for (int l = H.h_first[q]; l < H.h_first[q + 1]; ++l) {
         const int x = pos[H.h_list[l]];
-        DRec& d = H.h_recs[x];
-        const bool conn = d.type == 101 || d.type == 201;
+        const DRec& d = H.h_recs[x];
         if (!has_flux(d)) continue;
-        if (last >= 0 && !conn && H.h_recs[last].f == d.f) H.h_recs[last].next = x;
-        else if (!conn || d.owner) fr.push_back(x);
-        last = conn ? -1 : x;
+        sum |= d.f == face;
+        face = d.f;
+        slist.push_back(x);
+        if (!is_conn(d)) { fr.push_back(x); continue; }
+        const int g = giver[d.cf];
+        sum |= d.owner ? g != x : g < 0 || taker(g) != x;
+        if (g == x) fr.push_back(x);
       }
+      if (!sum) { slist.resize(at); continue; }
+      sfirst.push_back((int)at);
+      fr.resize(std::remove_if(fr.begin() + fat, fr.end(), [&](int x) { return !is_conn(H.h_recs[x]); }) - fr.begin());
     }
+    H.nsum = (int)sfirst.size();
+    for (int at : sfirst) sum_cells[p].push_back(slist[at]);
+    for (int x : slist) H.h_recs[x].summed = 1;
+    sfirst.push_back((int)slist.size());
+    CK(H.sfirst.alloc(sfirst.size()));
+    CK(H.slist.alloc(std::max<size_t>(slist.size(), 1)));
+    CK(cudaMemcpy(H.sfirst.p, sfirst.data(), sfirst.size() * sizeof(int), cudaMemcpyHostToDevice));
+    if (!slist.empty()) CK(cudaMemcpy(H.slist.p, slist.data(), slist.size() * sizeof(int), cudaMemcpyHostToDevice));
     // the record kernel's thread order: by block, face and whether it is a connection, then by cell, so that
     // the threads of a warp take the same branches and neighbouring cells
     std::stable_sort(fr.begin(), fr.end(), [&](int x, int y) {
@@ -1303,13 +1343,14 @@ int ice_gpu_set_records(ice_gpu_ctx* c, int32_t nrec, const int32_t* ri, const d
     CK(H.frec.alloc(std::max<size_t>(fr.size(), 1)));
     if (!fr.empty()) CK(cudaMemcpy(H.frec.p, fr.data(), fr.size() * sizeof(int), cudaMemcpyHostToDevice));
     CK(H.connF.alloc((size_t)std::max(ncf, 1) * H.nc));
+    CK(cudaMemset(H.connF.p, 0, (size_t)std::max(ncf, 1) * H.nc * sizeof(double)));
     if (int rc = upload_recs(c, H)) return rc;
   }
   // the boundary faces that a family leaves without a flux where another has one: its record kernel zeroes them
-  bool alike = true;                   // every family has the same codes face by face, and none an MK family's 200
+  bool alike = true;       // every family has the same codes face by face, none an MK family's 200 and no cell of k_cell_sum
   for (int p = 0; p < c->P.nfam && alike; ++p) {
     const std::vector<DRec>& x = c->fam[p].h_recs; const std::vector<DRec>& y = c->fam[0].h_recs;
-    alike = x.size() == y.size();
+    alike = x.size() == y.size() && c->fam[p].nsum == 0;
     for (size_t q = 0; q < x.size() && alike; ++q)
       alike = x[q].type == y[q].type && x[q].b == y[q].b && x[q].f == y[q].f && x[q].i == y[q].i && x[q].j == y[q].j &&
               x[q].k == y[q].k && x[q].type != 200;
@@ -1317,19 +1358,27 @@ int ice_gpu_set_records(ice_gpu_ctx* c, int32_t nrec, const int32_t* ri, const d
   for (int p = 0; p < c->P.nfam; ++p) c->fam[p].nzface = 0;
   if (!alike) {
     std::vector<std::vector<long long>> has(c->P.nfam);      // (place of the face) * 4 + direction
-    auto place = [&](const DRec& d) {
+    auto place = [&](const DRec& d, int f) {
       const DBlock& B = c->hblk[d.b];
-      const int dir = (d.f - 1) / 2;
-      const long long i = d.i + (dir == 0 && d.f % 2 == 0), j = d.j + (dir == 1 && d.f % 2 == 0),
-                      k = d.k + (dir == 2 && d.f % 2 == 0);
+      const int dir = (f - 1) / 2;
+      const long long i = d.i + (dir == 0 && f % 2 == 0), j = d.j + (dir == 1 && f % 2 == 0),
+                      k = d.k + (dir == 2 && f % 2 == 0);
       const long long ni = B.ni + (dir == 0), nj = B.nj + (dir == 1);
       return (B.foff[dir] + (k * nj + j) * ni + i) * 4 + dir;
     };
     std::vector<long long> all;
     for (int p = 0; p < c->P.nfam; ++p) {
       for (const DRec& d : c->fam[p].h_recs)
-        if (d.type != 0 && !(d.type == 200 && c->fam[p].closure == ICE_CLOSURE_MK)) has[p].push_back(place(d));
+        if (d.type != 0 && !(d.type == 200 && c->fam[p].closure == ICE_CLOSURE_MK)) has[p].push_back(place(d, d.f));
+      for (int x : sum_cells[p]) {               // k_cell_sum writes all of their boundary faces
+        const DRec& d = c->fam[p].h_recs[x];
+        const int* n = &c->dims[3 * d.b];
+        const int at[3] = {d.i, d.j, d.k};
+        for (int f = 1; f <= 6; ++f)
+          if (at[(f - 1) / 2] == (f % 2 == 1 ? 0 : n[(f - 1) / 2] - 1)) has[p].push_back(place(d, f));
+      }
       std::sort(has[p].begin(), has[p].end());
+      has[p].erase(std::unique(has[p].begin(), has[p].end()), has[p].end());
       all.insert(all.end(), has[p].begin(), has[p].end());
     }
     std::sort(all.begin(), all.end());

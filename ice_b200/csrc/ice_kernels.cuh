@@ -677,10 +677,10 @@ __global__ void k_ghost(Geo G, FamDev F, const DRec* recs, int nrec, int nrb, in
   }
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= nrec) return;
-  const DRec r = recs[n];
-  if (!stepped(G, r.b)) return;
-  if (layers & 1) ghost1_rec<CL>(G, F, r);
-  if (layers & 2) ghost2_rec<CL>(G, F, r);
+  const int run = recs[n].run;                   // a face listed more than once: its records in table order
+  if (!stepped(G, recs[n].b)) return;
+  if (layers & 1) for (int m = 0; m < run; ++m) ghost1_rec<CL>(G, F, recs[n + m]);
+  if (layers & 2) for (int m = 0; m < run; ++m) ghost2_rec<CL>(G, F, recs[n + m]);
 }
 
 // ------------------------------------------------------------------ boundary fluxes
@@ -733,16 +733,10 @@ __device__ __forceinline__ bool rec_face(const Geo& G, const FamDev& F, const DR
     }
     bf = (double)mn(bo, bq);
   }
-  bool bad = record_flux<CL, RS, LIM, R>(G, F, r, fl, conn ? &bf : nullptr);
-  for (int n = r.next; n >= 0; n = recs[n].next) {      // a table that lists a face twice: the sum
-    double more[nc];
-    bad |= record_flux<CL, RS, LIM, R>(G, F, recs[n], more, nullptr);
-#pragma unroll
-    for (int v = 0; v < nc; ++v) fl[v] = fl[v] + more[v];
-  }
-  put_flux<CL, R>(G, F, G.blk[r.b], r.f, r.i, r.j, r.k, fl, 1.0);
+  const bool bad = record_flux<CL, RS, LIM, R>(G, F, r, fl, conn ? &bf : nullptr);
+  if (!r.summed) put_flux<CL, R>(G, F, G.blk[r.b], r.f, r.i, r.j, r.k, fl, 1.0);
   if (conn) {
-    put_flux<CL, R>(G, F, G.blk[r.pb], r.pf, r.pi, r.pj, r.pk, fl, -1.0);
+    if (r.pf) put_flux<CL, R>(G, F, G.blk[r.pb], r.pf, r.pi, r.pj, r.pk, fl, -1.0);
     if (F.connF) {
 #pragma unroll
       for (int v = 0; v < nc; ++v) F.connF[(long long)r.cf * nc + v] = fl[v];
@@ -779,6 +773,51 @@ template <int CL, int RS, int LIM, typename R>
 __global__ void __launch_bounds__(128, 4) k_rec(Geo G, FamDev F, const DRec* recs, const int* frec, int nfrec, Status* st) {
   if (rec_thread<CL, RS, LIM, R>(G, F, recs, frec, nfrec, blockIdx.x * blockDim.x + threadIdx.x))
     atomicOr(&st->flags, (unsigned)ICE_GPU_ST_BAD_RECON);
+}
+
+// The cells of a table that lists one of their faces more than once, or a connection that is not one owner and its one
+// partner: every record of the cell in the order of faces and table (bound_cell, Mod_BC_Fluxes.f90:105-144), connections from
+// connF. Such a cell's boundary fluxes are wanted for their sum alone: it goes to the first of its boundary faces,
+// zeros to the others. parts = 3: what a float leaves of it to the next two (the FP32-flux form's 1-D runs, whose cells sum in
+// FP64 and have four faces or more there). Runs after the record and flux kernels and after a split run's exchange.
+template <int CL, int RS, typename R>
+__global__ void __launch_bounds__(128, 4) k_cell_sum(Geo G, FamDev F, const DRec* recs, const int* first, const int* list, int n,
+                                                     int parts, Status* st) {
+  constexpr int nc = NC<CL>::v;
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= n) return;
+  const DRec& o = recs[list[first[c]]];
+  if (!stepped(G, o.b)) return;
+  double acc[nc];
+#pragma unroll
+  for (int v = 0; v < nc; ++v) acc[v] = 0.0;
+  bool bad = false;
+  for (int m = first[c]; m < first[c + 1]; ++m) {
+    const DRec& r = recs[list[m]];
+    double fl[nc];
+    if (r.type == 101 || r.type == 201) {
+#pragma unroll
+      for (int v = 0; v < nc; ++v) { const double x = F.connF[(long long)r.cf * nc + v]; fl[v] = r.owner ? x : -x; }
+    } else {
+      bad |= record_flux<CL, RS, LIM_ANY, R>(G, F, r, fl, nullptr);
+    }
+#pragma unroll
+    for (int v = 0; v < nc; ++v) acc[v] = acc[v] + fl[v];
+  }
+  const DBlock& B = G.blk[o.b];
+  for (int f = 1; f <= 6; ++f) {
+    const int d = (f - 1) / 2, x = d == 0 ? o.i : d == 1 ? o.j : o.k, len = d == 0 ? B.ni : d == 1 ? B.nj : B.nk;
+    if (x != (f % 2 == 1 ? 0 : len - 1)) continue;
+    double part[nc];
+#pragma unroll
+    for (int v = 0; v < nc; ++v) {
+      part[v] = parts > 0 ? (double)(R)acc[v] : 0.0;
+      acc[v] = not_finite(part[v]) ? 0.0 : acc[v] - part[v];
+    }
+    put_flux<CL, R>(G, F, B, f, o.i, o.j, o.k, part, 1.0);
+    --parts;
+  }
+  if (bad) atomicOr(&st->flags, (unsigned)ICE_GPU_ST_BAD_RECON);
 }
 
 // The sum of a cell's boundary fluxes in face order: lo(d, v), hi(d, v) the fluxes of the faces below and above

@@ -44,8 +44,9 @@ struct DRec {                // one boundary record, 0-based cells
   int b, i, j, k, f, type;
   int bs, is, js, ks, fs;
   int owner, cf;             // cf 0-based (-1 when none)
-  int next;                  // another record of the same cell and face (place in the family's records), or -1
-  int pb, pi, pj, pk, pf;    // the partner's cell and its own face (connections; fs says where the ghosts come from)
+  int run;                   // among the ghost kernel's records: this one and those of the same face after it; 0 after the first
+  int pb, pi, pj, pk, pf;    // the partner's cell and its own face (connections; fs says where the ghosts come from), pf 0
+                             // where the owner's flux is not the partner's (k_cell_sum)
   int normal_dir;
   double massflux, velocity, alpha, beta, temperature, radius, gfixed;
   // host-computed once per record (the platform libm of the driver's host, as the
@@ -54,6 +55,7 @@ struct DRec {                // one boundary record, 0-based cells
   // chimera (102): donors cd0 .. cd0 + cn1 - 1 of ghost layer 1, then cn2 of layer 2, in the family's
   // donor arrays (FamDev::cdon, cw)
   int cd0, cn1, cn2;
+  int summed;                // k_cell_sum gives the cell's boundary faces
 };
 
 // The two ghost cells of a record that copies cells (0, 400, 101, 201), as places in a variable's pool: the first
@@ -114,7 +116,8 @@ struct FamDev {              // what the kernels of one family read
   double* tau;               // NI
   double* S;                 // [v][NI]: the stage's source (coupled runs)
   float* Sf;                 // the FP32-flux form's source, [v][NI] floats in the same buffer (else null)
-  double* connF;             // [ncf][nc]: a split run's connection fluxes on their way to and from other ranks
+  double* connF;             // [ncf][nc]: a split run's connection fluxes on their way to and from other ranks, and those
+                             // k_cell_sum reads (else null)
   void* Ff[3];               // the face fluxes of a stage [v][NF] per direction, in the form's precision; a face
                              // of the block's boundary holds its record's flux, zero where no record has one
   const ZeroFace* zface;     // the boundary faces without a flux that another family's stage gave one
@@ -163,6 +166,7 @@ struct LaunchArgs {
   int ghost_split;                                   // a record's second layer reads another's first
   const int* frec; int nfrec;                        // the records whose flux is computed, in thread order
   const SweepJob* fjobs; int nfjob;                  // the flux kernel's CTAs
+  const int* sfirst; const int* slist; int nsum;     // the cells of k_cell_sum and their records
   const Tile* tiles; int ntile; int TX, TY, KZ;     // the 1-D stage kernel's tiles
   bool own_source;                                   // the source has a kernel of its own
   const unsigned char* mlp_img;                      // the family's surrogate network (null: the plain closure)

@@ -50,6 +50,8 @@ void launch_flux_k(const LaunchArgs& a) {
     a.xchg(a, ICE_GPU_HALO_FLUX);
     if (a.nrec > 0) k_conn_in<CL, R><<<(a.nrec + 127) / 128, 128, 0, a.s>>>(a.G, a.F, a.recs, a.nrec);
   }
+  if (a.nsum > 0)
+    k_cell_sum<CL, RS, R><<<(a.nsum + 127) / 128, 128, 0, a.s>>>(a.G, a.F, a.recs, a.sfirst, a.slist, a.nsum, a.plane ? 3 : 1, a.st);
 }
 
 // The Jameson weights as the faces read them: in the precision of the fluxes, in FP64 for the plane kernel.
