@@ -63,12 +63,16 @@ struct HRec {
 
 template <typename T> struct DevBuf {
   T* p = nullptr; size_t n = 0;
+  bool on_host = false;                      // managed memory held on the host
   ~DevBuf() { if (p) cudaFree(p); }
   cudaError_t alloc(size_t count) {
     if (p) { cudaFree(p); p = nullptr; }
-    n = count;
+    n = 0; on_host = false;
     if (count == 0) return cudaSuccess;
-    return cudaMalloc((void**)&p, count * sizeof(T));
+    const cudaError_t e = cudaMalloc((void**)&p, count * sizeof(T));
+    if (e == cudaSuccess) n = count;
+    else { p = nullptr; cudaGetLastError(); }          // reported here, not by the next call's check
+    return e;
   }
   // For what can lie on the host at a price: where the device has no room left, managed memory held there, which
   // the kernels read and write over the bus: 5 steps of AG on 261 k cells in FP64 took 62 ms so, 19 with room (pages
@@ -76,14 +80,14 @@ template <typename T> struct DevBuf {
   cudaError_t alloc_or_managed(size_t count) {
     cudaError_t e = alloc(count);
     if (e != cudaErrorMemoryAllocation) return e;
-    cudaGetLastError();
-    p = nullptr;
     e = cudaMallocManaged((void**)&p, count * sizeof(T));
-    if (e != cudaSuccess) { p = nullptr; n = 0; return e; }
     int dev = 0;
-    if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
-    if ((e = cudaMemAdvise(p, count * sizeof(T), cudaMemAdviseSetPreferredLocation, cudaCpuDeviceId)) != cudaSuccess) return e;
-    return cudaMemAdvise(p, count * sizeof(T), cudaMemAdviseSetAccessedBy, dev);
+    if (e == cudaSuccess) e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaMemAdvise(p, count * sizeof(T), cudaMemAdviseSetPreferredLocation, cudaCpuDeviceId);
+    if (e == cudaSuccess) e = cudaMemAdvise(p, count * sizeof(T), cudaMemAdviseSetAccessedBy, dev);
+    if (e == cudaSuccess) { n = count; on_host = true; }
+    else { if (p) cudaFree(p); p = nullptr; cudaGetLastError(); }
+    return e;
   }
 };
 
@@ -258,6 +262,26 @@ static void free_graphs(ice_gpu_ctx* c) {
   for (auto& row : c->graph_fam) for (auto& g : row) if (g) { cudaGraphExecDestroy(g); g = nullptr; }
 }
 
+// Gives back the device memory of what a step makes again (ensure_flux): the metric rows, the face fluxes, the
+// FP32-flux form's weights. Between calls only: the next step's ensure_flux places them anew. False: nothing lay on the device.
+static bool yield_room(ice_gpu_ctx* c) {
+  bool any = (c->row.p && !c->row.on_host) || (c->flux.p && !c->flux.on_host);
+  for (int p = 0; p < c->P.nfam; ++p) any = any || (c->fam[p].betaf.p && !c->fam[p].betaf.on_host);
+  if (!any || cudaStreamSynchronize(c->stream) != cudaSuccess) return false;
+  free_graphs(c);
+  c->row.alloc(0); c->flux.alloc(0);
+  for (int p = 0; p < c->P.nfam; ++p) c->fam[p].betaf.alloc(0);
+  c->rows_ok = c->flux_ok = false;
+  c->flux_word = 0;
+  return true;
+}
+
+// Device memory for what has no place on the host, after create: the step's own work memory makes room for it.
+template <typename T> static cudaError_t with_room(ice_gpu_ctx* c, DevBuf<T>& b, size_t count) {
+  const cudaError_t e = b.alloc(count);
+  return e == cudaErrorMemoryAllocation && yield_room(c) ? b.alloc(count) : e;
+}
+
 // The surrogate source runs for family p: on, trained, a coupled run in the FP32-flux form.
 static bool sur_active(const ice_gpu_ctx* c, int p);
 
@@ -349,17 +373,17 @@ static int build_geo32(ice_gpu_ctx* c) {
   if (c->P.precision != ICE_PREC_FP32FLUX || c->geo32_ok) return 0;
   bool fresh = false;
   for (int d = 0; d < 3; ++d) {
-    if (!c->facef[d].p && c->NF[d] > 0) { CK(c->facef[d].alloc((size_t)c->NF[d])); fresh = true; }
+    if (!c->facef[d].p && c->NF[d] > 0) { CK(with_room(c, c->facef[d], (size_t)c->NF[d])); fresh = true; }
     if (c->NF[d] > 0) {
       k_face32<<<grid_of(c->NF[d]), 256, 0, c->stream>>>(c->face[d].p, c->NF[d], c->facef[d].p);
       CK(cudaGetLastError());
     }
   }
-  if (!c->dlf.p) { CK(c->dlf.alloc((size_t)3 * c->NR)); fresh = true; }
+  if (!c->dlf.p) { CK(with_room(c, c->dlf, (size_t)3 * c->NR)); fresh = true; }
   k_dl32<<<grid_of(3 * c->NR), 256, 0, c->stream>>>(c->dl.p, 3 * c->NR, c->dlf.p);
   CK(cudaGetLastError());
   if (c->P.coupled && c->gas.p) {
-    if (!c->gasf.p) { CK(c->gasf.alloc((size_t)9 * c->NI)); fresh = true; }
+    if (!c->gasf.p) { CK(with_room(c, c->gasf, (size_t)9 * c->NI)); fresh = true; }
     k_dl32<<<grid_of(9 * c->NI), 256, 0, c->stream>>>(c->gas.p, 9 * c->NI, c->gasf.p);
     CK(cudaGetLastError());
   }
@@ -413,7 +437,7 @@ __global__ void k_unpack_flux(double* __restrict__ F, int nc, const int4* __rest
 static int ensure_xbuf(ice_gpu_ctx* c, size_t n, cudaStream_t s) {
   if (c->xdev.n >= n && c->xhost_n >= n) return 0;
   CK(cudaStreamSynchronize(s));                    // the last exchange's copy and unpack read the buffers
-  if (c->xdev.n < n) CK(c->xdev.alloc(n));
+  if (c->xdev.n < n) CK(with_room(c, c->xdev, n));
   if (c->xhost_n < n) {
     if (c->xhost) cudaFreeHost(c->xhost);
     c->xhost = nullptr; c->xhost_n = 0;
@@ -421,6 +445,16 @@ static int ensure_xbuf(ice_gpu_ctx* c, size_t n, cudaStream_t s) {
     c->xhost_n = n;
   }
   return 0;
+}
+
+// The buffers for the largest exchange of a step, before the step's work memory takes its place.
+static int ensure_xbufs(ice_gpu_ctx* c) {
+  size_t n = 1;
+  if (c->owned.empty()) return 0;
+  for (int kind = 0; kind < 3; ++kind)
+    for (int p = 0; p < c->P.nfam; ++p)
+      n = std::max(n, (c->hs[kind][p].size() + c->hr[kind][p].size()) * (kind == ICE_GPU_HALO_BETA ? 1 : c->fam[p].nc) + 1);
+  return ensure_xbuf(c, n, c->stream);
 }
 
 // One exchange of a split step (Mod_GhostExchange.f90:737-800 for the cells), at its point of the
@@ -756,7 +790,7 @@ static int build_sweeps(ice_gpu_ctx* c) {
     std::vector<SweepJob> g(f.size());
     for (size_t q = 0; q < ord.size(); ++q) g[q] = f[ord[q]];
     H.nfjob = (int)g.size();
-    CK(H.fjobs.alloc(g.size()));
+    CK(with_room(c, H.fjobs, g.size()));
     if (!g.empty()) CK(cudaMemcpy(H.fjobs.p, g.data(), g.size() * sizeof(SweepJob), cudaMemcpyHostToDevice));
   }
   return 0;
@@ -813,7 +847,7 @@ static int build_tiles(ice_gpu_ctx* c) {
           for (int i = 0; i < ni; i += sx) t.push_back(Tile{b, i, j, k, 1});
     }
     c->ntile = (int)t.size();
-    CK(c->tiles.alloc(t.size()));
+    CK(with_room(c, c->tiles, t.size()));
     CK(cudaMemcpy(c->tiles.p, t.data(), t.size() * sizeof(Tile), cudaMemcpyHostToDevice));
   }
   if (int rc = build_sweeps(c)) return rc;
@@ -828,9 +862,9 @@ static int build_tiles(ice_gpu_ctx* c) {
     }
   }
   c->nchunk = (int)ch.size();
-  CK(c->chunks.alloc(ch.size()));
+  CK(with_room(c, c->chunks, ch.size()));
   CK(cudaMemcpy(c->chunks.p, ch.data(), ch.size() * sizeof(NormChunk), cudaMemcpyHostToDevice));
-  CK(c->npart.alloc((size_t)c->nchunk * 5));
+  CK(with_room(c, c->npart, (size_t)c->nchunk * 5));
   return 0;
 }
 
@@ -1019,7 +1053,7 @@ int ice_gpu_upload_state(ice_gpu_ctx* c, int32_t b1, int32_t p1, const double* p
   const DBlock& B = c->hblk[b1 - 1];
   FamHost& H = c->fam[p1 - 1];
   long long ng = (long long)(B.ni + 4) * (B.nj + 4) * (B.nk + 4);
-  if (!c->xfer.p) CK(c->xfer.alloc((size_t)c->ng_max * kMaxNC));
+  if (!c->xfer.p) CK(with_room(c, c->xfer, (size_t)c->ng_max * kMaxNC));
   CK(cudaStreamSynchronize(c->stream));
   CK(cudaMemcpyAsync(c->xfer.p, prim, (size_t)ng * H.nc * sizeof(double), cudaMemcpyHostToDevice, c->stream));
   k_aos2soa<<<grid_of(ng), 256, 0, c->stream>>>(c->xfer.p, H.S[c->phase].p + B.goff, c->NG, ng, H.nc,
@@ -1044,7 +1078,7 @@ int ice_gpu_download_state(ice_gpu_ctx* c, int32_t b1, int32_t p1, double* prim)
   FamHost& H = c->fam[p1 - 1];
   long long ng = (long long)(B.ni + 4) * (B.nj + 4) * (B.nk + 4);
   if (!prim) return fail(c, ICE_GPU_EINVAL, "download_state: null prim");
-  if (!c->xfer.p) CK(c->xfer.alloc((size_t)c->ng_max * kMaxNC));
+  if (!c->xfer.p) CK(with_room(c, c->xfer, (size_t)c->ng_max * kMaxNC));
   k_soa2aos<<<grid_of(ng), 256, 0, c->stream>>>(H.S[c->phase].p + B.goff, c->xfer.p, c->NG, ng, H.nc,
                                                  B.ni + 4, B.nj + 4, B.px);
   CK(cudaGetLastError());
@@ -1088,7 +1122,7 @@ int ice_gpu_update_params(ice_gpu_ctx* c, const ice_gpu_params* P) {
   if (P->irs && !c->P.irs) {
     for (int p = 0; p < c->P.nfam; ++p) {
       FamHost& H = c->fam[p];
-      CK(H.resid.alloc((size_t)H.nc * c->NI)); CK(H.resid2.alloc((size_t)H.nc * c->NI)); CK(H.resid3.alloc((size_t)H.nc * c->NI));
+      CK(with_room(c, H.resid, (size_t)H.nc * c->NI)); CK(with_room(c, H.resid2, (size_t)H.nc * c->NI)); CK(with_room(c, H.resid3, (size_t)H.nc * c->NI));
     }
   }
   CK(cudaStreamSynchronize(c->stream));
@@ -1109,7 +1143,7 @@ int ice_gpu_update_params(ice_gpu_ctx* c, const ice_gpu_params* P) {
 // record; the ghost kernel then runs as two launches, every record as it is.
 static int upload_recs(ice_gpu_ctx* c, FamHost& H) {
   const std::vector<DRec>& dr = H.h_recs;
-  CK(H.recs.alloc(dr.size()));
+  CK(with_room(c, H.recs, dr.size()));
   H.ghost_split = false;
   for (const DRec& r : dr) {
     if (r.type == 0 || r.type == 102) continue;
@@ -1164,8 +1198,8 @@ static int upload_recs(ice_gpu_ctx* c, FamHost& H) {
   ext.insert(ext.end(), copy.begin(), copy.end());
   H.ncopy = (int)ext.size();
   H.ngrec = (int)g.size();
-  CK(H.grecs.alloc(g.size()));
-  CK(H.gcopy.alloc(ext.size()));
+  CK(with_room(c, H.grecs, g.size()));
+  CK(with_room(c, H.gcopy, ext.size()));
   if (!g.empty()) CK(cudaMemcpy(H.grecs.p, g.data(), g.size() * sizeof(DRec), cudaMemcpyHostToDevice));
   if (!ext.empty()) CK(cudaMemcpy(H.gcopy.p, ext.data(), ext.size() * sizeof(GhostCopy), cudaMemcpyHostToDevice));
   return 0;
@@ -1217,6 +1251,7 @@ int ice_gpu_set_records(ice_gpu_ctx* c, int32_t nrec, const int32_t* ri, const d
     if ((t == 401 || t == 403) && r.massflux != 0.0 && !c->P.coupled)
       return fail(c, ICE_GPU_EINVAL, "record %d: inlet %d takes its speed from the gas, and the run has no gas", n + 1, t);
   }
+  c->have_records = false;                                // until the table is on the device whole
   std::vector<std::vector<int>> sum_cells(c->P.nfam);     // per family, a record of each cell of k_cell_sum
   for (int p = 0; p < c->P.nfam; ++p) {
     FamHost& H = c->fam[p];
@@ -1323,8 +1358,8 @@ int ice_gpu_set_records(ice_gpu_ctx* c, int32_t nrec, const int32_t* ri, const d
     for (int at : sfirst) sum_cells[p].push_back(slist[at]);
     for (int x : slist) H.h_recs[x].summed = 1;
     sfirst.push_back((int)slist.size());
-    CK(H.sfirst.alloc(sfirst.size()));
-    CK(H.slist.alloc(std::max<size_t>(slist.size(), 1)));
+    CK(with_room(c, H.sfirst, sfirst.size()));
+    CK(with_room(c, H.slist, std::max<size_t>(slist.size(), 1)));
     CK(cudaMemcpy(H.sfirst.p, sfirst.data(), sfirst.size() * sizeof(int), cudaMemcpyHostToDevice));
     if (!slist.empty()) CK(cudaMemcpy(H.slist.p, slist.data(), slist.size() * sizeof(int), cudaMemcpyHostToDevice));
     // the record kernel's thread order: by block, face and whether it is a connection, then by cell, so that
@@ -1340,9 +1375,9 @@ int ice_gpu_set_records(ice_gpu_ctx* c, int32_t nrec, const int32_t* ri, const d
       return a.i < b.i;
     });
     H.nfrec = (int)fr.size();
-    CK(H.frec.alloc(std::max<size_t>(fr.size(), 1)));
+    CK(with_room(c, H.frec, std::max<size_t>(fr.size(), 1)));
     if (!fr.empty()) CK(cudaMemcpy(H.frec.p, fr.data(), fr.size() * sizeof(int), cudaMemcpyHostToDevice));
-    CK(H.connF.alloc((size_t)std::max(ncf, 1) * H.nc));
+    CK(with_room(c, H.connF, (size_t)std::max(ncf, 1) * H.nc));
     CK(cudaMemset(H.connF.p, 0, (size_t)std::max(ncf, 1) * H.nc * sizeof(double)));
     if (int rc = upload_recs(c, H)) return rc;
   }
@@ -1389,7 +1424,7 @@ int ice_gpu_set_records(ice_gpu_ctx* c, int32_t nrec, const int32_t* ri, const d
         if (!std::binary_search(has[p].begin(), has[p].end(), x)) z.push_back(ZeroFace{x / 4, (int)(x % 4)});
       FamHost& H = c->fam[p];
       H.nzface = (int)z.size();
-      CK(H.zface.alloc(z.size()));
+      CK(with_room(c, H.zface, z.size()));
       if (!z.empty()) CK(cudaMemcpy(H.zface.p, z.data(), z.size() * sizeof(ZeroFace), cudaMemcpyHostToDevice));
     }
   }
@@ -1431,6 +1466,7 @@ int ice_gpu_set_chimera(ice_gpu_ctx* c, int32_t nrec, const int32_t* nchi, const
                   d[3], d[0]);
     if (!std::isfinite(weight[s])) return fail(c, ICE_GPU_EINVAL, "donor %lld: weight is not finite", s + 1);
   }
+  c->have_chimera = false;                                // until the donors are on the device whole
   for (int p = 0; p < c->P.nfam; ++p) {
     FamHost& H = c->fam[p];
     std::vector<int4> dn;
@@ -1446,8 +1482,8 @@ int ice_gpu_set_chimera(ice_gpu_ctx* c, int32_t nrec, const int32_t* nchi, const
       }
     }
     if (int rc = upload_recs(c, H)) return rc;
-    CK(H.cdon.alloc(std::max<size_t>(dn.size(), 1)));
-    CK(H.cw.alloc(std::max<size_t>(dw.size(), 1)));
+    CK(with_room(c, H.cdon, std::max<size_t>(dn.size(), 1)));
+    CK(with_room(c, H.cw, std::max<size_t>(dw.size(), 1)));
     if (!dn.empty()) {
       CK(cudaMemcpy(H.cdon.p, dn.data(), dn.size() * sizeof(int4), cudaMemcpyHostToDevice));
       CK(cudaMemcpy(H.cw.p, dw.data(), dw.size() * sizeof(double), cudaMemcpyHostToDevice));
@@ -1474,9 +1510,9 @@ int ice_gpu_set_imports(ice_gpu_ctx* c, int32_t b1, int32_t p1, const double* im
       if (!std::isfinite(imports[q])) return fail(c, ICE_GPU_EINVAL, "set_imports: a rate is not finite");
   CK(cudaStreamSynchronize(c->stream));
   if (!H.have_imp) {
-    CK(H.imp.alloc((size_t)c->NI * H.nc));
+    CK(with_room(c, H.imp, (size_t)c->NI * H.nc));
     CK(cudaMemset(H.imp.p, 0, (size_t)c->NI * H.nc * sizeof(double)));
-    CK(H.escan.alloc(1));
+    CK(with_room(c, H.escan, 1));
     H.have_imp = true;
     free_graphs(c);
   }
@@ -1497,7 +1533,7 @@ int ice_gpu_set_exchange(ice_gpu_ctx* c, int32_t on) {
   if (on && !c->exchange)
     for (int p = 0; p < c->P.nfam; ++p) {
       FamHost& H = c->fam[p];
-      CK(H.xstep.alloc((size_t)5 * c->NI));
+      CK(with_room(c, H.xstep, (size_t)5 * c->NI));
       CK(cudaMemset(H.xstep.p, 0, (size_t)5 * c->NI * sizeof(double)));
     }
   c->exchange = on != 0;
@@ -1553,6 +1589,7 @@ int ice_gpu_step(ice_gpu_ctx* c, int32_t nsteps, ice_gpu_step_out* out) {
   if (!c) return ICE_GPU_EINVAL;
   if (int rc = check_ready(c)) return rc;
   if (int rc = build_geo32(c)) return rc;
+  if (int rc = ensure_xbufs(c)) return rc;
   if (int rc = ensure_flux(c)) return rc;
   if (nsteps < 0) return fail(c, ICE_GPU_EINVAL, "step: nsteps %d", nsteps);
   cudaStream_t s = c->stream;
@@ -1660,7 +1697,7 @@ int ice_gpu_step_host(ice_gpu_ctx* c, int32_t nsteps, const double* const* prim_
     const long long ng = (long long)(B.ni + 4) * (B.nj + 4) * (B.nk + 4);
     for (int p = 0; p < nf; ++p) off[(size_t)b * nf + p + 1] = off[(size_t)b * nf + p] + ng * c->fam[p].nc;
   }
-  if (c->xall.n < (size_t)off.back()) CK(c->xall.alloc((size_t)off.back()));
+  if (c->xall.n < (size_t)off.back()) CK(with_room(c, c->xall, (size_t)off.back()));
   if (int rc = ensure_flux(c)) return rc;        // after xall: the fluxes can do without device memory
   if (!c->s_up) CK(cudaStreamCreateWithFlags(&c->s_up, cudaStreamNonBlocking));
   if (!c->s_down) CK(cudaStreamCreateWithFlags(&c->s_down, cudaStreamNonBlocking));
@@ -1796,14 +1833,17 @@ int ice_gpu_set_partition(ice_gpu_ctx* c, const int32_t* owned) {
     for (int b = 0; b < c->nb; ++b) { o[b] = owned[b] != 0; n += o[b]; }
     if (n == 0) return fail(c, ICE_GPU_EINVAL, "set_partition: this rank steps no block");
     c->owned = o;
-    CK(c->owned_dev.alloc(c->nb));
+    CK(with_room(c, c->owned_dev, c->nb));
     CK(cudaMemcpy(c->owned_dev.p, o.data(), c->nb, cudaMemcpyHostToDevice));
   }
   CK(cudaStreamSynchronize(c->stream));
   free_graphs(c);
+  const bool had = c->have_records;
+  c->have_records = false;                                   // until the tables are on the device again
   for (int p = 0; p < c->P.nfam; ++p)
     if (int rc = upload_recs(c, c->fam[p])) return rc;       // the ghost copies are of the stepped blocks
   if (build_tiles(c)) return ICE_GPU_ECUDA;
+  c->have_records = had;
   return 0;
 }
 
@@ -1834,8 +1874,8 @@ int ice_gpu_set_halo(ice_gpu_ctx* c, int32_t kind, int32_t p1, int32_t nsend, co
   }
   c->hs[kind][p] = lists[0];
   c->hr[kind][p] = lists[1];
-  CK(c->hs_dev[kind][p].alloc(lists[0].size()));
-  CK(c->hr_dev[kind][p].alloc(lists[1].size()));
+  CK(with_room(c, c->hs_dev[kind][p], lists[0].size()));
+  CK(with_room(c, c->hr_dev[kind][p], lists[1].size()));
   if (!lists[0].empty())
     CK(cudaMemcpy(c->hs_dev[kind][p].p, lists[0].data(), lists[0].size() * sizeof(int4), cudaMemcpyHostToDevice));
   if (!lists[1].empty())
@@ -1875,8 +1915,8 @@ int ice_gpu_surrogate_train(ice_gpu_ctx* c, int32_t p1, const ice_gpu_surrogate_
     return fail(c, ICE_GPU_EINVAL, "surrogate_train: options out of range");
   FamHost& H = c->fam[p1 - 1];
   DevBuf<float> X, T;
-  CK(X.alloc((size_t)o->nsamples * MLP_IN));
-  CK(T.alloc((size_t)o->nsamples * 2));
+  CK(with_room(c, X, (size_t)o->nsamples * MLP_IN));
+  CK(with_room(c, T, (size_t)o->nsamples * 2));
   FamDev F = make_famdev(c, p1 - 1, 1, c->phase);
   if (mlp_make_samples(H.closure, make_geo(c), F, c->P.drag, c->P.heat, c->P.blow, o->nsamples, o->seed, o->jitter,
                        X.p, T.p, c->stream))
@@ -1884,11 +1924,15 @@ int ice_gpu_surrogate_train(ice_gpu_ctx* c, int32_t p1, const ice_gpu_surrogate_
   MlpTrainOpts to{o->nsamples, o->epochs, o->batch, o->lr, o->jitter, o->seed, o->val_frac};
   MlpTrainReport tr{};
   std::string err;
-  if (mlp_train(X.p, T.p, o->nsamples, to, H.mlp_w, H.mlp_norm, tr, c->stream, err))
-    return fail(c, ICE_GPU_ECUDA, "%s: %s", err.c_str(), cudaGetErrorString(cudaGetLastError()));
+  for (int again = 0;; ++again) {
+    if (!mlp_train(X.p, T.p, o->nsamples, to, H.mlp_w, H.mlp_norm, tr, c->stream, err)) break;
+    const cudaError_t e = cudaGetLastError();
+    if (again == 0 && e == cudaErrorMemoryAllocation && yield_room(c)) continue;
+    return fail(c, ICE_GPU_ECUDA, "%s: %s", err.c_str(), cudaGetErrorString(e));
+  }
   std::vector<unsigned char> img;
   mlp_image(H.mlp_w.data(), img);
-  CK(H.mlp_img.alloc(img.size()));
+  CK(with_room(c, H.mlp_img, img.size()));
   CK(cudaMemcpy(H.mlp_img.p, img.data(), img.size(), cudaMemcpyHostToDevice));
   H.sur_on = true;
   free_graphs(c);
