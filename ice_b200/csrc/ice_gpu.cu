@@ -796,11 +796,11 @@ static int build_sweeps(ice_gpu_ctx* c) {
   return 0;
 }
 
-// What a step keeps beyond its states and inputs: the metric rows (after a block's metrics) and the face fluxes,
-// the largest family's, in the word of the running form; the faces no record gives a flux are zero and stay so
-// (before the first step, after a change of form, after a new boundary table). 96 + 12 nc (24 nc) bytes a cell
-// in 3-D, allocated last and, on a device that the rest fills, in managed memory: such a run is slower, not
-// refused.
+// What a step keeps beyond its states and inputs: the metric rows (after a block's metrics), the face fluxes,
+// the largest family's, in the word of the running form, and the FP32-flux form's weights; the faces no record gives a flux
+// are zero and stay so (after a change of form, after a new boundary table). 96 + 12 nc (24 nc) bytes a cell
+// in 3-D. Made when the blocks and the table are complete (setup_work), so that the first step does not pay for
+// them; on a device that the rest fills, in managed memory: such a run is slower, not refused.
 static int ensure_flux(ice_gpu_ctx* c) {
   if (!c->rows_ok) {
     if (!c->row.p) CK(c->row.alloc_or_managed((size_t)12 * c->NI));
@@ -809,6 +809,12 @@ static int ensure_flux(ice_gpu_ctx* c) {
     c->rows_ok = true;
   }
   const int word = sweeps64(c) ? 8 : 4;
+  if (word == 4 && c->P.shock_detector && !plane(c))
+    for (int p = 0; p < c->P.nfam; ++p)
+      if (!c->fam[p].betaf.p) {
+        CK(c->fam[p].betaf.alloc_or_managed(c->NI));
+        free_graphs(c);
+      }
   if (c->flux_ok && c->flux_word == word) return 0;
   size_t nc = 0;
   for (int p = 0; p < c->P.nfam; ++p) nc = std::max(nc, (size_t)c->fam[p].nc);
@@ -824,14 +830,15 @@ static int ensure_flux(ice_gpu_ctx* c) {
     CK(c->flux.alloc_or_managed(n));
   }
   CK(cudaMemsetAsync(c->flux.p, 0, n, c->stream));
-  for (int p = 0; p < c->P.nfam; ++p)
-    if (word == 4 && c->P.shock_detector && !c->fam[p].betaf.p) {
-      CK(c->fam[p].betaf.alloc_or_managed(c->NI));
-      free_graphs(c);
-    }
   c->flux_word = word;
   c->flux_ok = true;
   return 0;
+}
+
+// After a block's metrics or a boundary table: a step's work memory, once both are complete.
+static int setup_work(ice_gpu_ctx* c) {
+  if (!c->have_records || !std::all_of(c->have_block.begin(), c->have_block.end(), [](bool x) { return x; })) return 0;
+  return ensure_flux(c);
 }
 
 static int build_tiles(ice_gpu_ctx* c) {
@@ -995,6 +1002,7 @@ int ice_gpu_set_block(ice_gpu_ctx* c, int32_t b1, const double* f1, const double
   const double* fs[3] = {f1, f2, f3};
   long long nf[3] = {(long long)(ni + 1) * nj * nk, (long long)ni * (nj + 1) * nk, (long long)ni * nj * (nk + 1)};
   std::vector<double> tmp;
+  CK(cudaStreamSynchronize(c->stream));             // the rows of the metrics before these
   for (int d = 0; d < 3; ++d) {
     tmp.resize(nf[d]);
     for (int comp = 0; comp < 4; ++comp) {
@@ -1018,10 +1026,12 @@ int ice_gpu_set_block(ice_gpu_ctx* c, int32_t b1, const double* f1, const double
     }
     CK(cudaMemcpy(c->M.p + (long long)comp * c->NI + B.ioff, tmp.data(), ncell * sizeof(double), cudaMemcpyHostToDevice));
   }
-  CK(cudaStreamSynchronize(c->stream));
+  CK(cudaStreamSynchronize(cudaStreamLegacy));      // the copies, which the stream's kernels do not wait for
   c->have_block[b1 - 1] = true;
   c->geo32_ok = false;
-  c->rows_ok = false;
+  if (!c->rows_ok) return setup_work(c);
+  k_rows<<<grid_of(ncell), 256, 0, c->stream>>>(c->M.p, c->row.p, c->NI, B.ioff, ncell);     // new metrics of one block
+  CK(cudaGetLastError());
   return 0;
 }
 
@@ -1128,7 +1138,6 @@ int ice_gpu_update_params(ice_gpu_ctx* c, const ice_gpu_params* P) {
   CK(cudaStreamSynchronize(c->stream));
   c->P = *P;
   for (int p = 0; p < c->P.nfam; ++p) c->fam[p].riemann = P->fam[p].riemann;
-  c->flux_ok = false;                  // the form or the sensor may have changed
   free_graphs(c);
   return 0;
 }
@@ -1434,7 +1443,7 @@ int ice_gpu_set_records(ice_gpu_ctx* c, int32_t nrec, const int32_t* ri, const d
   c->have_chimera = c->nchim == 0;
   c->have_records = true;
   free_graphs(c);
-  return 0;
+  return setup_work(c);
 }
 
 // The donors of the table's chimera records (ICE_bc_type%ni, donorID, volume_fraction,
