@@ -50,20 +50,24 @@ ICE_DIV_FN unsigned ice_div_hi(double x) {
 /* 2^-200 <= |x| < 2^200: x is a dividend of the quotients below (and zero is one). */
 ICE_DIV_FN int ice_div_in(double x) { return ice_div_hi(x) - (823u << 20) < (400u << 20); }
 
-/* The low words that no divisor has (see above). */
+/* The low words of the divisors with j <= 2^14. */
 #define ICE_DIV_LOW 0xffffc000u
 
-/* x is a divisor of the quotients below: the same range, and its low word is below ICE_DIV_LOW. */
-ICE_DIV_FN int ice_div_by(double x) {
+ICE_DIV_FN unsigned ice_div_lo(double x) {
 #ifdef __CUDA_ARCH__
-  const unsigned lo = (unsigned)__double2loint(x);
+  return (unsigned)__double2loint(x);
 #else
   union { double d; unsigned long long u; } v;
   v.d = x;
-  const unsigned lo = (unsigned)v.u;
+  return (unsigned)v.u;
 #endif
-  return ice_div_in(x) && lo < ICE_DIV_LOW;
 }
+
+/* j <= 2^14 */
+ICE_DIV_FN int ice_div_top(double x) { return ice_div_lo(x) >= ICE_DIV_LOW && (~ice_div_hi(x) & 0xfffffu) == 0u; }
+
+/* x is a divisor of the quotients below: the same range, and by its low word not one with j <= 2^14. */
+ICE_DIV_FN int ice_div_by(double x) { return ice_div_in(x) && ice_div_lo(x) < ICE_DIV_LOW; }
 
 /* The first approximation of 1/b (rcp.approx.ftz.f64 on the device; its error: see above). */
 ICE_DIV_FN double ice_div_seed(double b) {
