@@ -746,12 +746,13 @@ static int build_sweeps(ice_gpu_ctx* c) {
   int dev = 0;
   CK(cudaGetDevice(&dev));
   CK(cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, dev));
-  const bool f64 = c->P.precision != ICE_PREC_FP32FLUX;
+  const bool f64 = sweeps64(c);
   for (int p = 0; p < c->P.nfam; ++p) {
     FamHost& H = c->fam[p];
     const TuneRow tr = tune_of(H.closure);
-    const int occ = H.closure == ICE_CLOSURE_AG ? (f64 ? SweepOcc<AG, double>::flux : SweepOcc<AG, float>::flux)
-                                                : (f64 ? SweepOcc<MK, double>::flux : SweepOcc<MK, float>::flux);
+    const int occ = H.closure == ICE_CLOSURE_AG   ? (f64 ? SweepOcc<AG, double>::flux : SweepOcc<AG, float>::flux)
+                    : H.closure == ICE_CLOSURE_IG ? (f64 ? SweepOcc<IG, double>::flux : SweepOcc<IG, float>::flux)
+                                                  : (f64 ? SweepOcc<MK, double>::flux : SweepOcc<MK, float>::flux);
     const double slots = (double)c->nsm * occ * SW_NT;
     // groups of SW_XC cells an x CTA takes: the start of a CTA (its job, its block, their loads) is a chain of its
     // own, 183 / 172 us for one / four groups (FP32 IG, 128 x 126 x 129); one in a run too small for two waves
