@@ -40,8 +40,6 @@
 #include <string>
 #include <algorithm>
 #include <memory>
-#include <queue>
-#include <functional>
 #include "ice_kernels.cuh"
 #include "ice_sweep.cuh"
 #include "ice_mlp.cuh"
@@ -626,10 +624,14 @@ static void enqueue_step(ice_gpu_ctx* c, int phase, cudaStream_t s, void (*tick)
 // ones that leave half of the issue slots free. The families share the face fluxes, so their faces stay one
 // after the other. Three families on 8 blocks of 1.7 M cells, 8 steps in the FP32-flux form: 32.8 ms in one
 // branch, 31.4 in two; 4 blocks of 0.35 M cells, 5 steps in FP64: 12.3 and 11.5, 10.8 with the sources under the
-// faces. One family takes the second branch while a cell a thread is less than four waves: AG cells of 28 k
-// 1.83 / 1.69 ms (20 steps, FP32 form) and 261 k 8.47 / 8.35 (10 steps, FP64) gain, 885 k 9.88 / 10.04 lose.
+// faces. One family takes the second branch while a cell a thread is less than four waves in FP64, one and a half in
+// the FP32-flux form, whose faces leave less idle. ms of 6 steps in one branch and in two, by thousands of cells:
+//   FP32, evaporating: AG 30 0.528 / 0.496, 79 0.842 / 0.810, 125 1.097 / 1.115, 175 1.468 / 1.510, 300 2.18 / 2.24; IG 125 0.745 / 0.717
+//   FP64: AG evaporating 30 1.21 / 0.96, 262 5.02 / 4.91, 342 6.39 / 6.24, 884 14.55 / 14.40; IG inert 175 1.93 / 1.86, 342 3.05 / 3.03,
+//   884 6.51 / 6.56, 1,727 12.07 / 12.14
 static bool two_branches(const ice_gpu_ctx* c) {
-  return c->P.nfam > 1 || (own_source(c, 0) && c->NI < 4LL * 4 * SW_NT * c->nsm);
+  const long long wave = 4LL * SW_NT * c->nsm;
+  return c->P.nfam > 1 || (own_source(c, 0) && 2 * c->NI < (sweeps64(c) ? 8 : 3) * wave);
 }
 
 static cudaError_t capture_step(ice_gpu_ctx* c, int phase, cudaStream_t s) {
