@@ -17,7 +17,7 @@
 //                  connections as on-device copies in one HBM pool    (Lib_Ghost.f90:29-387)
 //     k_beta       Jameson sensor (when on)                           (Mod_Fluxes.f90:366-389)
 //     k_flux       the fluxes of the boundary records (Mod_BC_Fluxes.f90:105-170) and of the interior faces
-//                  (Mod_Fluxes.f90:599-685)
+//                  (Mod_Fluxes.f90:599-685); k_cell_sum where the table lists a face of a cell more than once
 //     k_cells      the cells' update: a cell's boundary faces, then its interior faces in the odd-then-even
 //                  order (Mod_Fluxes.f90:421-521), the source (in the FP32-flux form evaluated here for a family
 //                  without evaporation: Mod_Sources.f90:465-622), the residual

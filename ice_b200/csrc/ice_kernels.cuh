@@ -890,7 +890,7 @@ __global__ void __launch_bounds__(256, 4) k_source(Geo G, FamDev F) {
 #endif
 template <int CL, int RS, int LIM, typename R>
 __global__ void __launch_bounds__(256, ICE_STAGE_MINB)
-k_stage(Geo G, FamDev F, const Tile* tiles, int TX, int TY, int KZ, int write_r, Status* st) {
+k_stage(Geo G, FamDev F, const Tile* tiles, int TX, int TY, int KZ, Status* st) {
   constexpr int nc = NC<CL>::v;
   extern __shared__ double smem[];
   const int NT = TX * TY;
@@ -1012,7 +1012,7 @@ k_stage(Geo G, FamDev F, const Tile* tiles, int TX, int TY, int KZ, int write_r,
       double s[nc];
 #pragma unroll
       for (int v = 0; v < nc; ++v)
-        s[v] = !F.coupled ? 0.0 : F.Sf ? (double)F.Sf[(long long)v * G.NI + q] : F.S[(long long)v * G.NI + q];
+        s[v] = F.coupled ? (double)F.Sf[(long long)v * G.NI + q] : 0.0;
       if (F.xstep) accumulate_source<CL>(F.xstep, G.NI, q, s, F.xfirst, F.rk);
       const double dt = F.dt ? F.dt[q] : *F.dtg;
       const double vol = G.vol[q];
@@ -1024,26 +1024,19 @@ k_stage(Geo G, FamDev F, const Tile* tiles, int TX, int TY, int KZ, int write_r,
       }
 #pragma unroll
       for (int v = 0; v < nc; ++v) if (F.frozen_mask & (1u << v)) r[v] = 0.0;
-      if (write_r) {
+      double po[nc], co[nc], cn[nc];
 #pragma unroll
-        for (int v = 0; v < nc; ++v) F.resid[(long long)v * G.NI + q] = r[v];
-      } else {
-        double po[nc], co[nc], cn[nc];
+      for (int v = 0; v < nc; ++v) po[v] = F.U0[(long long)v * G.NG + g];
+      prim2cons<CL, double>(po, co, F.mat.cp);
+      prim2cons<CL, double>(p, cn, F.mat.cp);
 #pragma unroll
-        for (int v = 0; v < nc; ++v) po[v] = F.U0[(long long)v * G.NG + g];
-        prim2cons<CL, double>(po, co, F.mat.cp);
-        prim2cons<CL, double>(p, cn, F.mat.cp);
+      for (int v = 0; v < nc; ++v) { double rr = (cn[v] - co[v] + r[v]) * F.rk; cn[v] = co[v] + rr; }
+      if (cn[0] < 0.0) atomicAdd(&st->nfloored, 1ULL);
+      cons2prim<CL>(cn, p, F.mat.cp);
+      if (F.realize && realize<CL>(p)) atomicAdd(&st->nrealized, 1ULL);
+      if (!check_prim<CL, double>(p)) atomicOr(&st->flags, (unsigned)ICE_GPU_ST_NAN_STATE);
 #pragma unroll
-        for (int v = 0; v < nc; ++v) { double rr = (cn[v] - co[v] + r[v]) * F.rk; cn[v] = co[v] + rr; }
-        if (cn[0] < 0.0) atomicAdd(&st->nfloored, 1ULL);
-        cons2prim<CL>(cn, p, F.mat.cp);
-        if constexpr (sizeof(R) == 4) {
-          if (F.realize && realize<CL>(p)) atomicAdd(&st->nrealized, 1ULL);
-        }
-        if (!check_prim<CL, double>(p)) atomicOr(&st->flags, (unsigned)ICE_GPU_ST_NAN_STATE);
-#pragma unroll
-        for (int v = 0; v < nc; ++v) F.Uo[(long long)v * G.NG + g] = p[v];
-      }
+      for (int v = 0; v < nc; ++v) F.Uo[(long long)v * G.NG + g] = p[v];
     }
     __syncthreads();
     double* tmp = flo; flo = fhi; fhi = tmp;

@@ -20,8 +20,7 @@ void launch_stage_k(const LaunchArgs& a, bool write_r) {
         cudaFuncSetAttribute(k_stage<CL, RS, LIM_ANY, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, 98304);
         attr = true;
       }
-      k_stage<CL, RS, LIM_ANY, R><<<a.ntile, a.TX * a.TY, sh, a.s>>>(a.G, a.F, a.tiles, a.TX, a.TY, a.KZ,
-                                                                     write_r ? 1 : 0, a.st);
+      k_stage<CL, RS, LIM_ANY, R><<<a.ntile, a.TX * a.TY, sh, a.s>>>(a.G, a.F, a.tiles, a.TX, a.TY, a.KZ, a.st);
       return;
     }
   }
