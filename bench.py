@@ -113,10 +113,18 @@ def algorithmic_bytes(case, precision: int = abi.PREC_FP64) -> float:
     return float(np.mean(per))
 
 
+# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per cell of one stage's flux and cell kernels, the mean of
+# the three RK stages, from an ncu capture of the 4-block case of the 48-block tree in the chosen form (3,714,802 cells).
+# The 48-block case is the same recipe, so its stages move about the same bytes per cell.
+DRAM_BYTES_PER_CELL = {"MK": 520.0, "IG": 574.6, "AG": 927.6}
+
+
 def dram_traffic(case, workload: str, precision: int):
     """Measured DRAM bytes of one stage of the workload (mean over its families), where a capture of the same
     recipe and form exists; None otherwise."""
-    return None
+    if not workload.startswith("multiblock") or precision != abi.PREC_FP32FLUX:
+        return None
+    return float(np.mean([DRAM_BYTES_PER_CELL[f.closure] for f in case.families])) * case.ncells
 
 
 class Clocks:
