@@ -60,7 +60,7 @@ struct DRec {                // one boundary record, 0-based cells
 
 // The two ghost cells of a record that copies cells (0, 400, 101, 201), as places in a variable's pool: the first
 // layer g1 takes m, the second g2 takes p (a 400 record 3 g1 - 3 m + p); code 0 has no second (g2 = kNoGhost).
-// Sixteen bytes in place of a record's two hundred. A pool has fewer than 2^32 places: three buffers of six
+// Sixteen bytes in place of a record's 192. A pool has fewer than 2^32 places: three buffers of six
 // doubles for each are more than the GPU holds.
 struct GhostCopy { unsigned m, p, g1, g2; };
 constexpr unsigned kNoGhost = 0xffffffffu;

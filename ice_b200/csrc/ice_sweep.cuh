@@ -17,12 +17,12 @@
 // dealt out to the threads and the update behind a barrier moved 24 nc bytes per cell and stage, but took the
 // registers and shared memory of all its phases at once: one CTA of 6 to 8 warps per SM in FP64 (20 % of the
 // issue slots, dependent FP64 chains), two in FP32 (49 %), DRAM at 5 and 16 % of peak. Here the faces need
-// 128 registers or fewer and no barrier, every direction is in flight at once, and the fluxes cost
+// 72 to 128 registers (168 for AG in FP64) and no barrier, every direction is in flight at once, and the fluxes cost
 // 6 nc words per cell of bandwidth that stood idle. FP64: the two divisions of every limited slope
 // run branchless and side by side (ice_div.h), where a compiled division's branch ordered them one after the
-// other. Stage kernels, the one kernel (+ records) / k_flux + k_cells (one B200, CUDA events): FP64 IG
-// 96 x 95 x 97 967 / 212 + 74 us, AG 64 x 61 x 67 693 + 161 / 146 + 49 us; FP32 form IG 128 x 126 x 129
-// 516 + 28 / 173 + 139 us, AG 96^3 387 + 30 / 152 + 105 us.
+// other. The one kernel (+ records; CUDA events) / k_flux + k_cells (the profiler's launch times), one B200: FP64 IG
+// 96 x 95 x 97 967 / 215 + 63 us, AG 64 x 61 x 67 693 + 161 / 142 + 39 us; FP32 form IG 128 x 126 x 129
+// 516 + 28 / 168 + 136 us, AG 96^3 387 + 30 / 146 + 98 us.
 #pragma once
 #include "ice_kernels.cuh"
 

@@ -29,7 +29,7 @@ from ice_b200 import abi, configs  # noqa: E402
 from ice_b200.solver import Solver  # noqa: E402
 
 CLOSURES = ("MK", "IG", "AG")
-KZ = (8, 16, 24, 32)
+KZ = (4, 8, 16, 32)
 ZPASS = (2, 4, 8)
 WCAP = {"MK": (4, 8, 16), "IG": (4, 8, 16), "AG": (4, 8, 16)}
 KC_STAGE = 4
@@ -54,7 +54,7 @@ def header(rows: dict, table: dict, what: str) -> str:
              "//",
              "//   kz     the longest march of a thread along y or z, in faces (shorter where the run is small: choose_march)",
              "//   zpass  the start of a march (the slope of its first cell), in thirds of a face: the larger, the longer",
-             "//          the marches a small run takes",
+             "//          the marches, of a run of more threads than the GPU holds (below that every march is one face)",
              "//   wcap   the planes of a slab, whose x, y and z faces run one after the other",
              "//",
              "// The environment variable ICE_GPU_TUNE=\"kz,zpass,wcap\" overrides the row of every closure (the",
